@@ -676,11 +676,13 @@ int plc_create(const plc_params *prm, const double *h_dzf_global, int device, pl
     if ((e = fft_set_lines(c, c->fft_lines_xf, c->fft_lines_x, c->fft_lines_y)) != cudaSuccess)
       return fail(cuda_status(c, e, "fft_set_lines"));
   }
-  // PLC_TRID = "tile" / "stream" pins the Thomas sweep (columns on chip or
-  // streamed through HBM) instead of timing both
+  // PLC_TRID = "split" / "tile" / "stream" pins the Thomas sweep (columns split
+  // over the threads of a block where they fit, on chip, or streamed through
+  // HBM; columns too tall for the split one are streamed under its pin)
   if (const char *env = getenv("PLC_TRID")) {
-    if (strcmp(env, "tile") != 0 && strcmp(env, "stream") != 0)
+    if (strcmp(env, "split") != 0 && strcmp(env, "tile") != 0 && strcmp(env, "stream") != 0)
       return fail(set_error(c, PLC_ERR_ARG, std::string("invalid PLC_TRID: ") + env));
+    c->trid_split = strcmp(env, "split") == 0;
     c->trid_tile = strcmp(env, "tile") == 0;
     c->trid_pinned = true;
   }

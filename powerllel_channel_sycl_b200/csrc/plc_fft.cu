@@ -3200,9 +3200,10 @@ cudaError_t fft_autotune_t(plc_ctx *c, T *const *f, size_t dev_max, int sms) {
          else
            return launch_fft_x_fwd(c, u, v, w, spec, s);
        });
-  // the Thomas sweep: on chip or streaming, timed on the spectral array (the
-  // choice changes speed, never results)
-  if (c->nx % 32 == 0 && !c->trid_pinned) {
+  // the Thomas sweep of columns too tall for the split one: on chip or
+  // streaming, timed on the spectral array (the choice changes speed, never
+  // results)
+  if (c->nx % 32 == 0 && !c->trid_pinned && !trid_split_ok(c->nz)) {
     float t_tile = -1.f, t_stream = -1.f;
     c->trid_tile = true;
     t_tile = time_of([&]() -> cudaError_t { return launch_trid(c, spec, s); });
@@ -3248,6 +3249,9 @@ static bool trid_tile_ok(const plc_ctx *c, size_t elem) {
   return c->trid_tile && c->nx % 32 == 0 && trid_tile_smem(c->nz, elem) <= c->trid_smem_max;
 }
 cudaError_t launch_trid(const plc_ctx *c, double *var, cudaStream_t s) {
+  if (c->trid_split && trid_split_ok(c->nz) &&
+      reinterpret_cast<unsigned long long>(var) % (2 * sizeof(double)) == 0)
+    return launch_trid_split(c, var, s);
   const long long plane = (long long)c->nx * c->ny;
   if (trid_tile_ok(c, sizeof(double))) {
     k_trid_tile<<<(unsigned)(plane / 32), 32, trid_tile_smem(c->nz, sizeof(double)), s>>>(
@@ -3260,6 +3264,9 @@ cudaError_t launch_trid(const plc_ctx *c, double *var, cudaStream_t s) {
   return cudaGetLastError();
 }
 cudaError_t launch_trid(const plc_ctx *c, float *var, cudaStream_t s) {
+  if (c->trid_split && trid_split_ok(c->nz) &&
+      reinterpret_cast<unsigned long long>(var) % (2 * sizeof(float)) == 0)
+    return launch_trid_split(c, var, s);
   const long long plane = (long long)c->nx * c->ny;
   if (trid_tile_ok(c, sizeof(float))) {
     k_trid_mixed_tile<<<(unsigned)(plane / 32), 32, trid_tile_smem(c->nz, sizeof(float)), s>>>(
@@ -3627,8 +3634,8 @@ cudaError_t batch_autotune(plc_ctx *const *cs, int n, cudaStream_t s, BatchPlan 
       bp->dir[dir].push_back(best);
     }
   }
-  // the Thomas sweep: streamed, or with the columns on chip (as the channels
-  // have it where PLC_TRID pins it)
+  // the Thomas sweep where a channel does not have the split one: streamed, or
+  // with the columns on chip (as the channels have it where PLC_TRID pins it)
   bp->trid_tile = false;
   bool trid_pinned = false, trid_tiles = true;
   for (int m = 0; m < n; ++m) {
@@ -3637,7 +3644,7 @@ cudaError_t batch_autotune(plc_ctx *const *cs, int n, cudaStream_t s, BatchPlan 
   }
   if (trid_pinned) {
     bp->trid_tile = trid_tiles && trid_tile_batch_ok(cs, n);
-  } else if (trid_tile_batch_ok(cs, n)) {
+  } else if (!trid_split_batch_ok(cs, n) && trid_tile_batch_ok(cs, n)) {
     const float ts = time_of([&]() { return launch_trid_batch(cs, n, false, s); });
     const float tt = time_of([&]() { return launch_trid_batch(cs, n, true, s); });
     bp->trid_tile = tt >= 0.f && (ts < 0.f || tt < ts);
@@ -3675,6 +3682,7 @@ bool trid_tile_batch_ok(plc_ctx *const *cs, int n) {
 }
 
 cudaError_t launch_trid_batch(plc_ctx *const *cs, int n, bool tile, cudaStream_t s, bool pdl) {
+  if (trid_split_batch_ok(cs, n)) return launch_trid_split_batch(cs, n, s, pdl);
   if (tile && trid_tile_batch_ok(cs, n)) {
     for (int q0 = 0; q0 < n; q0 += kBatchMax) {
       TrtBatch b;

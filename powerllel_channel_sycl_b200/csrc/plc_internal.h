@@ -108,10 +108,13 @@ struct plc_ctx {
   int fft_plan_x = 0, fft_plan_y = 0;
   // family of the forward x transform (-1: that of the backward one)
   int fft_plan_xf = -1;
-  // Thomas sweep with the columns on chip (else the streaming sweep), chosen
-  // by the autotuner; the device's shared-memory limit per block
+  // Thomas sweep: its columns split over the threads of a block wherever they fit
+  // (trid_split_ok), unless PLC_TRID pins a serial one; taller columns have
+  // the sweep with the columns on chip or the streaming one, as the autotuner
+  // finds; the device's shared-memory limit per block
+  bool trid_split = true;
   bool trid_tile = true;
-  bool trid_pinned = false;  // PLC_TRID = "tile" or "stream"
+  bool trid_pinned = false;  // PLC_TRID = "split", "tile" or "stream"
   // z planes per block of the RK stages (0: the kernels' maximum), chosen by
   // the autotuner among kRkChunks; PLC_RK_KCHUNK pins it
   int rk_kchunk = 0;
@@ -252,6 +255,12 @@ cudaError_t launch_fft_y(const plc_ctx *c, float *var, bool inverse,
                          cudaStream_t s);
 cudaError_t launch_trid(const plc_ctx *c, double *var, cudaStream_t s);
 cudaError_t launch_trid(const plc_ctx *c, float *var, cudaStream_t s);
+// the sweep with each column split over the threads of a block (plc_trid.cu),
+// for columns of trid_split_ok(nz) planes; spectral arrays not aligned to a
+// pair of elements take the streaming sweep
+bool trid_split_ok(int nz);
+cudaError_t launch_trid_split(const plc_ctx *c, double *var, cudaStream_t s);
+cudaError_t launch_trid_split(const plc_ctx *c, float *var, cudaStream_t s);
 cudaError_t launch_check(const plc_ctx *c, const double *u, const double *v,
                          const double *w, int what, cudaStream_t s);
 cudaError_t launch_check(const plc_ctx *c, const float *u, const float *v,
@@ -340,6 +349,9 @@ cudaError_t launch_fft_y_batch(plc_ctx *const *cs, int n, bool inverse, const Ba
                                const cudaStream_t *ss, int ns);
 cudaError_t launch_trid_batch(plc_ctx *const *cs, int n, bool tile, cudaStream_t s,
                               bool pdl = false);
+// the batched split sweep, and whether every channel uses it
+cudaError_t launch_trid_split_batch(plc_ctx *const *cs, int n, cudaStream_t s, bool pdl);
+bool trid_split_batch_ok(plc_ctx *const *cs, int n);
 // whether every channel admits the batched on-chip Thomas sweep
 bool trid_tile_batch_ok(plc_ctx *const *cs, int n);
 cudaError_t launch_fft_x_bwd_batch(plc_ctx *const *cs, int n, const BatchPlan *bp,
