@@ -181,8 +181,9 @@ int plc_fft_plans(const plc_ctx *ctx, int *plan_x, int *plan_y);
  * timed separately from the backward one.  No counterpart in the reference. */
 int plc_fft_plan_x_fwd(const plc_ctx *ctx, int *plan);
 /* z planes per block of the two RK stages, timed per context at creation
- * among 8, 16, 24 and 32 (at most nz) on both fused stages; PLC_RK_KCHUNK
- * (FP64 form) and PLC_RK_KCHUNK_F32 (mixed form) pin it.  The choice changes speed; results only in the mixed form, whose
+ * among 8, 16, 24 and 32 (at most nz) on both fused stages (on a grid whose
+ * 8-plane blocks do not fill the device, a block may take a half or a quarter
+ * of them); PLC_RK_KCHUNK (FP64 form) and PLC_RK_KCHUNK_F32 (mixed form) pin it.  The choice changes speed; results only in the mixed form, whose
  * RK2 sums the bulk mean per block in FP32 (by FP32 rounding).  No
  * counterpart in the reference. */
 int plc_rk_kchunk(const plc_ctx *ctx, int *kchunk);

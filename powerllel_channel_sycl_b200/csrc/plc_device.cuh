@@ -108,6 +108,31 @@ static __device__ __noinline__ void store_images(T *q, const Geo &g, HaloCol h, 
   }
 }
 
+// The same image and ghost writes inline, for kernels in which a whole warp
+// takes them when one of its lanes has an image or the plane is a wall plane:
+// the image stores are predicated per lane, the ghost writes uniform per
+// plane.
+template <class T>
+static __device__ __forceinline__ void store_images_inline(T *q, const Geo &g, const HaloCol &h,
+                                                           long long c, int k, T v, int kind,
+                                                           T bc) {
+  if (h.dx) q[c + h.dx] = v;
+  if (h.dy) {
+    q[c + h.dy] = v;
+    if (h.dx) q[c + (h.dx + h.dy)] = v;
+  }
+  if (k == 1 || k == g.nz) {
+    T gv;
+    if (kind == BC_CENTRED)
+      gv = T(2) * bc - v;
+    else if (kind == BC_FACE)
+      gv = bc;
+    else
+      gv = v;
+    store_col(q, k == 1 ? c - g.XY : c + g.XY, h, gv);
+  }
+}
+
 // The same writes as store_with_halo for the point at halo'd index c of
 // column h, plane k.
 template <class T>

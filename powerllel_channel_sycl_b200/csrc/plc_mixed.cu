@@ -366,8 +366,11 @@ __global__ void __launch_bounds__(RX *TY, (STAGE == 2 && C2) ? 3 : 4)
     }
   }
   ZFace fa_c{}, fb_c{};  // z-face terms carried from plane k-1 (rows a, b)
-  const HaloCol ha = halo_col(g, i, ja), hb = halo_col(g, i, jb);
-  const bool xy_edge = (ha.dx | ha.dy | hb.dx | hb.dy) != 0;  // images in x or y
+  // a warp takes the image path as a whole when one of its lanes has images: no
+  // divergence between two paths and no call (boundary tiles set the time of
+  // a small grid)
+  const bool edge_w = __any_sync(0xffffffffu, i == 1 || i == g.nx || ja == 1 || ja == g.ny ||
+                                                  jb == g.ny);
   const int o = (2 * ty + 1) * HX + (tx + 1);  // point a in a slot
   int sm = 0, s0 = 1, sp = 2;                  // slots of planes k-1, k, k+1
   for (int k = kb; k <= ke; ++k) {
@@ -449,14 +452,16 @@ __global__ void __launch_bounds__(RX *TY, (STAGE == 2 && C2) ? 3 : 4)
             msum[d] = fmaf(x, dzl, msum[d]);
           }
       }
-      if (FUSE && (xy_edge || k == 1 || k == g.nz)) {
-        store_point(ou, g, ha, c, k, va[0], BC_CENTRED, bc_u);
-        store_point(ov, g, ha, c, k, va[1], BC_CENTRED, 0.f);
-        store_point(ow, g, ha, c, k, va[2], BC_FACE, 0.f);
+      if (FUSE && (edge_w || k == 1 || k == g.nz)) {
+        // (evaluated here: no registers held over the march)
+        const HaloCol ha = halo_col(g, i, ja), hb = halo_col(g, i, jb);
+        store_point_inline(ou, g, ha, c, k, va[0], BC_CENTRED, bc_u);
+        store_point_inline(ov, g, ha, c, k, va[1], BC_CENTRED, 0.f);
+        store_point_inline(ow, g, ha, c, k, va[2], BC_FACE, 0.f);
         if (act_b) {
-          store_point(ou, g, hb, c + X, k, vb[0], BC_CENTRED, bc_u);
-          store_point(ov, g, hb, c + X, k, vb[1], BC_CENTRED, 0.f);
-          store_point(ow, g, hb, c + X, k, vb[2], BC_FACE, 0.f);
+          store_point_inline(ou, g, hb, c + X, k, vb[0], BC_CENTRED, bc_u);
+          store_point_inline(ov, g, hb, c + X, k, vb[1], BC_CENTRED, 0.f);
+          store_point_inline(ow, g, hb, c + X, k, vb[2], BC_FACE, 0.f);
         }
       } else {  // no image or ghost to write
         ou[c] = va[0];
@@ -916,7 +921,7 @@ unsigned convert_blocks(const plc_ctx *c, long long n) {
 // Blocks of the FP32 RK grid at the smallest z chunk the autotuner may
 // choose (the capacity of the bulk-mean partials).
 long long rk32_blocks(const plc_ctx *c) {
-  const int kchunk = c->nz < kRkChunks[0] ? c->nz : kRkChunks[0];
+  const int k0 = kRkChunks[0] / kRkCutMax, kchunk = c->nz < k0 ? c->nz : k0;
   return (long long)((c->nx + RX - 1) / RX) * ((c->ny + RY - 1) / RY) *
          ((c->nz + kchunk - 1) / kchunk);
 }

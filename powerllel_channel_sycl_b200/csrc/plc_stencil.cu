@@ -418,7 +418,12 @@ size_t rk_tma_smem_bytes() {
   return (size_t)3 * NSLOT * SLOT * 8 + KCHUNK_TMA * sizeof(ZMetric) + 2 * NSLOT * 8 + 128;
 }
 
-template <int STAGE, bool FUSE, bool CRF>
+// INL: how the halo images are written.  Inline, a warp with an image lane taking
+// the image path as a whole: RK1 everywhere (768 x 384 x 256 0.86 -> 0.83 ms, 128 x
+// 64 x 64 25 -> 22 us) and RK2 of small grids, whose time the boundary tiles set
+// (162 x 108 x 90 50 -> 46 us).  Out of line, off the common path: RK2 of the others,
+// where the inline code cost it registers (1.08 -> 1.18 ms).
+template <int STAGE, bool FUSE, bool CRF, bool INL>
 __global__ void __launch_bounds__(RX *TY, 2)
     k_rk_tma(const __grid_constant__ CUtensorMap mu, const __grid_constant__ CUtensorMap mv,
              const __grid_constant__ CUtensorMap mw, Geo g, const StepConst *__restrict__ sc,
@@ -498,8 +503,11 @@ __global__ void __launch_bounds__(RX *TY, 2)
       bb[2] = ow[c + X];
     }
   }
-  const HaloCol ha = halo_col(g, i, ja), hb = halo_col(g, i, jb);
-  const bool xy_edge = (ha.dx | ha.dy | hb.dx | hb.dy) != 0;  // images in x or y
+  // !INL: the images of the two columns, held over the march
+  const HaloCol ha_o = halo_col(g, i, ja), hb_o = halo_col(g, i, jb);
+  const bool xy_edge = (ha_o.dx | ha_o.dy | hb_o.dx | hb_o.dy) != 0;  // images in x or y
+  const bool edge_w = INL && __any_sync(0xffffffffu, i == 1 || i == g.nx || ja == 1 ||
+                                                         ja == g.ny || jb == g.ny);
   const int o = (2 * ty + 1) * HX + (tx + 1);                 // point a in a slot
   int sm = 0, s0 = 1, sp = 2;                                 // slots of planes k-1, k, k+1
   for (int k = kb; k <= ke; ++k) {
@@ -568,14 +576,35 @@ __global__ void __launch_bounds__(RX *TY, 2)
           vb[d] = (qb[d] + dt * fb[d] + bb[d]) * 0.5;
         }
       }
-      if (FUSE && (xy_edge || k == 1 || k == g.nz)) {
-        store_point(ou, g, ha, c, k, va[0], BC_CENTRED, 0.0 - u_crf);
-        store_point(ov, g, ha, c, k, va[1], BC_CENTRED, 0.0);
-        store_point(ow, g, ha, c, k, va[2], BC_FACE, 0.0);
+      if constexpr (INL) {
+        if (FUSE && k == g.nz) va[2] = vb[2] = 0.0;  // w(nz) is the wall value
+        ou[c] = va[0];
+        ov[c] = va[1];
+        ow[c] = va[2];
         if (act_b) {
-          store_point(ou, g, hb, c + X, k, vb[0], BC_CENTRED, 0.0 - u_crf);
-          store_point(ov, g, hb, c + X, k, vb[1], BC_CENTRED, 0.0);
-          store_point(ow, g, hb, c + X, k, vb[2], BC_FACE, 0.0);
+          ou[c + X] = vb[0];
+          ov[c + X] = vb[1];
+          ow[c + X] = vb[2];
+        }
+        if (FUSE && (edge_w || k == 1 || k == g.nz)) {
+          const HaloCol ha = halo_col(g, i, ja), hb = halo_col(g, i, jb);
+          store_images_inline(ou, g, ha, c, k, va[0], BC_CENTRED, 0.0 - u_crf);
+          store_images_inline(ov, g, ha, c, k, va[1], BC_CENTRED, 0.0);
+          store_images_inline(ow, g, ha, c, k, va[2], BC_FACE, 0.0);
+          if (act_b) {
+            store_images_inline(ou, g, hb, c + X, k, vb[0], BC_CENTRED, 0.0 - u_crf);
+            store_images_inline(ov, g, hb, c + X, k, vb[1], BC_CENTRED, 0.0);
+            store_images_inline(ow, g, hb, c + X, k, vb[2], BC_FACE, 0.0);
+          }
+        }
+      } else if (FUSE && (xy_edge || k == 1 || k == g.nz)) {
+        store_point(ou, g, ha_o, c, k, va[0], BC_CENTRED, 0.0 - u_crf);
+        store_point(ov, g, ha_o, c, k, va[1], BC_CENTRED, 0.0);
+        store_point(ow, g, ha_o, c, k, va[2], BC_FACE, 0.0);
+        if (act_b) {
+          store_point(ou, g, hb_o, c + X, k, vb[0], BC_CENTRED, 0.0 - u_crf);
+          store_point(ov, g, hb_o, c + X, k, vb[1], BC_CENTRED, 0.0);
+          store_point(ow, g, hb_o, c + X, k, vb[2], BC_FACE, 0.0);
         }
       } else {  // no image or ghost to write
         ou[c] = va[0];
@@ -1487,14 +1516,31 @@ cudaError_t launch_rk_tma(const plc_ctx *c, const CUtensorMap &mu, const CUtenso
                           cudaStream_t s) {
   const int kchunk = rk_chunk(c, KCHUNK_TMA);
   dim3 grid((c->nx + RX - 1) / RX, (c->ny + RY - 1) / RY, (c->nz + kchunk - 1) / kchunk);
-  if (u_crf != 0.0)
-    k_rk_tma<STAGE, FUSE, true><<<grid, RX * TY, rk_tma_smem_bytes(), s>>>(
-        mu, mv, mw, c->geo(), c->d_sc, u_crf, ou, ov, ow, kchunk, c->d_err,
-        STAGE == 2 ? c->order[SK_RK2] : 0);
-  else
-    k_rk_tma<STAGE, FUSE, false><<<grid, RX * TY, rk_tma_smem_bytes(), s>>>(
-        mu, mv, mw, c->geo(), c->d_sc, u_crf, ou, ov, ow, kchunk, c->d_err,
-        STAGE == 2 ? c->order[SK_RK2] : 0);
+  auto go = [&](auto CRF, auto INL) {
+    k_rk_tma<STAGE, FUSE, decltype(CRF)::value, decltype(INL)::value>
+        <<<grid, RX * TY, rk_tma_smem_bytes(), s>>>(mu, mv, mw, c->geo(), c->d_sc, u_crf, ou, ov,
+                                                    ow, kchunk, c->d_err,
+                                                    STAGE == 2 ? c->order[SK_RK2] : 0);
+  };
+  // without the halo writes the two kernels are the same
+  const bool inl = FUSE && (STAGE == 1 || rk_small_grid(c));
+  const std::true_type yes{};
+  const std::false_type no{};
+  if constexpr (FUSE) {
+    if (inl) {
+      if (u_crf != 0.0)
+        go(yes, yes);
+      else
+        go(no, yes);
+      return cudaGetLastError();
+    }
+  }
+  if constexpr (!FUSE || STAGE == 2) {
+    if (u_crf != 0.0)
+      go(yes, no);
+    else
+      go(no, no);
+  }
   return cudaGetLastError();
 }
 
@@ -1505,18 +1551,20 @@ cudaError_t launch_rk_tma(const plc_ctx *c, const CUtensorMap &mu, const CUtenso
 cudaError_t rk_tma_configure() {
   const int bytes = (int)rk_tma_smem_bytes();
   cudaError_t e = cudaSuccess;
-#define PLC_RK_ATTR(S, F, C)                                                                \
-  if (e == cudaSuccess)                                                                     \
-    e = cudaFuncSetAttribute(k_rk_tma<S, F, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+#define PLC_RK_ATTR(S, F, C, I)                                                                \
+  if (e == cudaSuccess)                                                                        \
+    e = cudaFuncSetAttribute(k_rk_tma<S, F, C, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                              bytes);
-  PLC_RK_ATTR(1, true, true)
-  PLC_RK_ATTR(1, true, false)
-  PLC_RK_ATTR(1, false, true)
-  PLC_RK_ATTR(1, false, false)
-  PLC_RK_ATTR(2, true, true)
-  PLC_RK_ATTR(2, true, false)
-  PLC_RK_ATTR(2, false, true)
-  PLC_RK_ATTR(2, false, false)
+  PLC_RK_ATTR(1, true, true, true)
+  PLC_RK_ATTR(1, true, false, true)
+  PLC_RK_ATTR(1, false, true, false)
+  PLC_RK_ATTR(1, false, false, false)
+  PLC_RK_ATTR(2, true, true, true)
+  PLC_RK_ATTR(2, true, false, true)
+  PLC_RK_ATTR(2, true, true, false)
+  PLC_RK_ATTR(2, true, false, false)
+  PLC_RK_ATTR(2, false, true, false)
+  PLC_RK_ATTR(2, false, false, false)
 #undef PLC_RK_ATTR
   return e;
 }
