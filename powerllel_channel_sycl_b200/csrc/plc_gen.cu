@@ -536,8 +536,34 @@ void gen_free(plc_gen *gn) {
   if (gn->stream) cudaStreamDestroy(gn->stream);
 }
 
-// forward convolution and input gradient: the tcgen05 kernel, 128 voxels x
-// all output channels per block
+// dynamic shared memory that a block may take
+constexpr size_t kSmemMax = 226 * 1024;
+
+// Output channels per block of a halo-tile convolution: the most (of N and the
+// parts of it that are multiples of 16) of which two blocks fit an SM and whose
+// blocks fill the device -- fewer channels read the input tile again --, else
+// the fewest if one block fits, else 0.
+int halo_channels(Shape s, int ci, int n) {
+  const long long tiles = (long long)((s.Y * (s.X + 2) + kHaloM - 1) / kHaloM) * s.B * s.Z;
+  int least = 0;
+  for (int parts = 1; parts <= n / 16; ++parts) {
+    if (n % parts || n / parts % 16) continue;
+    const int nb = n / parts;
+    if (halo_smem(s.X, ci, nb) <= kSmemMax / 2 && tiles * parts >= 148) return nb;
+    if (halo_smem(s.X, ci, nb) <= kSmemMax) least = nb;
+  }
+  return least;
+}
+
+template <int NB>
+cudaError_t conv_halo(plc_gen *gn, Shape s, const bf16 *x, const bf16 *w, float *y, int ci, int n) {
+  const int tiles = (s.Y * (s.X + 2) + kHaloM - 1) / kHaloM;
+  k_conv3d_halo<NB><<<dim3((unsigned)(tiles * s.B * s.Z), (unsigned)(n / NB)), kHaloThreads,
+                      halo_smem(s.X, ci, NB), gn->stream>>>(s, x, w, y, ci, n, tiles, gn->derr);
+  return cudaGetLastError();
+}
+
+// the im2col kernel, 128 voxels x all output channels per block
 template <int N>
 cudaError_t conv_tc(plc_gen *gn, Shape s, const bf16 *x, const bf16 *w, float *y, int ci) {
   const unsigned gx = (unsigned)((s.voxels() + kTcM - 1) / kTcM);
@@ -545,8 +571,26 @@ cudaError_t conv_tc(plc_gen *gn, Shape s, const bf16 *x, const bf16 *w, float *y
   return cudaGetLastError();
 }
 
+// Forward convolution and input gradient: over halo tiles, or im2col where a
+// plane of the tile does not fit the shared memory (the same sums either way).
 int conv(plc_gen *gn, Shape s, const bf16 *x, const bf16 *w, float *y, int ci, int co) {
   cudaError_t e;
+  bool done = true;
+  switch (halo_channels(s, ci, co)) {
+    case 16: e = conv_halo<16>(gn, s, x, w, y, ci, co); break;
+    case 32: e = conv_halo<32>(gn, s, x, w, y, ci, co); break;
+    case 48: e = conv_halo<48>(gn, s, x, w, y, ci, co); break;
+    case 64: e = conv_halo<64>(gn, s, x, w, y, ci, co); break;
+    case 80: e = conv_halo<80>(gn, s, x, w, y, ci, co); break;
+    case 96: e = conv_halo<96>(gn, s, x, w, y, ci, co); break;
+    case 112: e = conv_halo<112>(gn, s, x, w, y, ci, co); break;
+    case 128: e = conv_halo<128>(gn, s, x, w, y, ci, co); break;
+    default: done = false; break;
+  }
+  if (done) {
+    GEN_CUDA(gn, e);
+    return PLC_OK;
+  }
   switch (co) {
     case 16: e = conv_tc<16>(gn, s, x, w, y, ci); break;
     case 32: e = conv_tc<32>(gn, s, x, w, y, ci); break;
@@ -567,6 +611,22 @@ cudaError_t conv_configure() {
   auto one = [&](auto kern, size_t bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
+  one(k_conv3d_halo<16>, kSmemMax);
+  one(k_conv3d_halo<32>, kSmemMax);
+  one(k_conv3d_halo<48>, kSmemMax);
+  one(k_conv3d_halo<64>, kSmemMax);
+  one(k_conv3d_halo<80>, kSmemMax);
+  one(k_conv3d_halo<96>, kSmemMax);
+  one(k_conv3d_halo<112>, kSmemMax);
+  one(k_conv3d_halo<128>, kSmemMax);
+  one(k_conv3d_wgrad_halo<16>, kSmemMax);
+  one(k_conv3d_wgrad_halo<32>, kSmemMax);
+  one(k_conv3d_wgrad_halo<48>, kSmemMax);
+  one(k_conv3d_wgrad_halo<64>, kSmemMax);
+  one(k_conv3d_wgrad_halo<80>, kSmemMax);
+  one(k_conv3d_wgrad_halo<96>, kSmemMax);
+  one(k_conv3d_wgrad_halo<112>, kSmemMax);
+  one(k_conv3d_wgrad_halo<128>, kSmemMax);
   one(k_conv3d_tc<16>, tc_smem_bytes<16>());
   one(k_conv3d_tc<32>, tc_smem_bytes<32>());
   one(k_conv3d_tc<48>, tc_smem_bytes<48>());
@@ -595,23 +655,59 @@ int check_device_error(plc_gen *gn) {
   return PLC_OK;
 }
 
+// The voxels of a weight gradient split over blocks: about 8 blocks per SM over
+// the 27 taps of the per-tap kernel, at least 16 voxels each.
+struct WgradSplit {
+  long long splits, chunk;
+  explicit WgradSplit(long long M) {
+    splits = std::max(1ll, std::min((long long)(148 * 8) / 27 + 1, (M + 15) / 16));
+    chunk = ((M + splits - 1) / splits + 15) / 16 * 16;
+    splits = (M + chunk - 1) / chunk;
+  }
+};
+
 template <int N>
 cudaError_t wgrad_tc(plc_gen *gn, Shape s, const bf16 *dy, const bf16 *x, float *dw, int co) {
-  const long long M = s.voxels();
-  // about 8 blocks per SM over the 27 taps, at least 16 voxels each
-  long long splits = std::max(1ll, std::min((long long)(148 * 8) / 27 + 1, (M + 15) / 16));
-  long long chunk = (M + splits - 1) / splits;
-  chunk = (chunk + 15) / 16 * 16;
-  splits = (M + chunk - 1) / chunk;
+  const auto [splits, chunk] = WgradSplit(s.voxels());
   k_conv3d_wgrad_tc<N><<<dim3((unsigned)splits, 1, 27), 128, tc_smem_bytes<N, kWgG, kWgNB>(), gn->stream>>>(
       s, dy, x, dw, co, chunk, gn->derr);
   return cudaGetLastError();
 }
 
-// weight gradient on the tensor cores: M = co (zero-padded to 128), N = ci
+// Halo tiles where rows are whole groups of 8 voxels and planes of 16, with the
+// split of the voxels of wgrad_tc; false elsewhere.
+template <int CO>
+bool wgrad_halo(plc_gen *gn, Shape s, const bf16 *dy, const bf16 *x, float *dw, int ci,
+                cudaError_t *e) {
+  const size_t smem = wg_smem<CO>(s.X);
+  if (s.X % 8 || (s.Y * s.X) % 16 || smem > kSmemMax) return false;
+  const WgradSplit w(s.voxels());
+  k_conv3d_wgrad_halo<CO><<<dim3((unsigned)w.splits, (unsigned)((3 * ci + 127) / 128 * 3)),
+                            kHaloThreads, smem, gn->stream>>>(s, dy, x, dw, ci, w.chunk, gn->derr);
+  *e = cudaGetLastError();
+  return true;
+}
+
+// weight gradient on the tensor cores: over halo tiles, else per tap with
+// M = co (zero-padded to 128), N = ci
 int wgrad(plc_gen *gn, Shape s, const bf16 *dy, const bf16 *x, float *dw, int ci, int co) {
   if (co > 128 || co % 16) return gen_error(gn, PLC_ERR_ARG, "weight gradient: co must be a multiple of 16 <= 128");
   cudaError_t e;
+  bool done = false;
+  switch (co) {
+    case 16: done = wgrad_halo<16>(gn, s, dy, x, dw, ci, &e); break;
+    case 32: done = wgrad_halo<32>(gn, s, dy, x, dw, ci, &e); break;
+    case 48: done = wgrad_halo<48>(gn, s, dy, x, dw, ci, &e); break;
+    case 64: done = wgrad_halo<64>(gn, s, dy, x, dw, ci, &e); break;
+    case 80: done = wgrad_halo<80>(gn, s, dy, x, dw, ci, &e); break;
+    case 96: done = wgrad_halo<96>(gn, s, dy, x, dw, ci, &e); break;
+    case 112: done = wgrad_halo<112>(gn, s, dy, x, dw, ci, &e); break;
+    case 128: done = wgrad_halo<128>(gn, s, dy, x, dw, ci, &e); break;
+  }
+  if (done) {
+    GEN_CUDA(gn, e);
+    return PLC_OK;
+  }
   switch (ci) {
     case 16: e = wgrad_tc<16>(gn, s, dy, x, dw, co); break;
     case 32: e = wgrad_tc<32>(gn, s, dy, x, dw, co); break;

@@ -456,5 +456,391 @@ __global__ void __launch_bounds__(128) k_conv3d_wgrad_tc(Shape s, const bf16 *__
   }
 }
 
+// ===========================================================================
+// Convolution and weight gradient over halo tiles.
+//
+// The kernels above copy the im2col rows of every tap, 27 reads of each input
+// value from L2, which is what bounded them (64 -> 32 channels on 4 x 64 x 48 x 64
+// voxels: 0.91 ms forward, 2.07 ms weight gradient; here 0.39 and 0.83).  Here a plane (b, z) is
+// numbered by padded positions p = y * (X + 2) + x + 1: the neighbour at (dz,
+// dy, dx) of the output at p is the input at p + dy * (X + 2) + dx of plane
+// z + dz, for every p whose x is not one of the two padding columns.  A tile of
+// consecutive positions therefore needs one run of consecutive rows of three
+// planes, and with the rows of a group of 8 channels 16 bytes apart in shared
+// memory a tap is only another start address of the UMMA operand.  Outputs at
+// padding positions are computed and dropped (2 of X + 2).
+// ===========================================================================
+
+// Row q of a halo tile whose first output position is p0: its voxel within the
+// plane, periodic in y and x (rows that only padding outputs read map to some
+// voxel of the plane).
+__device__ __forceinline__ int halo_voxel(const Shape &s, int p0, int q) {
+  const int XP = s.X + 2;
+  const int pos = p0 - (XP + 1) + q + 2 * XP;  // not negative; two rows up
+  int y = pos / XP;
+  int x = pos - y * XP - 1;
+  y = (y - 2) % s.Y;
+  y = y < 0 ? y + s.Y : y;
+  x = x < 0 ? s.X - 1 : (x >= s.X ? 0 : x);
+  return y * s.X + x;
+}
+
+// Low word of a UMMA shared-memory descriptor without swizzle: start address and
+// leading byte offset (K-major: between the K halves; MN-major: between the
+// 8-voxel groups of K), both in units of 16 bytes; the start address of
+// shared memory never carries out of its 14 bits, so that a neighbouring operand
+// is one 32-bit addition away.  High word: stride byte offset (K-major: between
+// 8-row groups; MN-major: between 8-channel groups) in the same units.
+__device__ __forceinline__ unsigned tc_desc_lo(unsigned saddr, unsigned lbo16) {
+  return (saddr >> 4) | (lbo16 << 16);
+}
+__device__ __forceinline__ unsigned tc_desc_hi(unsigned sbo16) { return sbo16 | (1u << 14); }
+// (one thread issues every MMA of a block one after another: the descriptors
+// cost it a few instructions each, not the twenty of assembling them anew)
+__device__ __forceinline__ void tc_mma(unsigned d, unsigned a_lo, unsigned a_hi, unsigned b_lo,
+                                       unsigned b_hi, unsigned idesc, unsigned acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, {%7, %7, %7, %7}, p;\n\t}"
+      :
+      : "r"(d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc), "r"(0u));
+}
+__device__ __forceinline__ void tc_commit(unsigned long long *bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                   tc_smem_u32(bar))
+               : "memory");
+}
+__device__ __forceinline__ void tc_ld16(unsigned addr, unsigned (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+      "%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(addr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+constexpr int tc_cols(int n) { return n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : (n <= 256 ? 256 : 512))); }
+
+constexpr int kHaloThreads = 256;
+constexpr int kHaloM = 256;  // positions of a convolution tile: two MMA tiles of 128
+
+// rows of a convolution's halo tile, = 2 (mod 4): the two rows and four channel
+// groups that 8 lanes copy together fall on different banks
+__host__ __device__ inline int halo_rows(int X) {
+  const int r = kHaloM + 2 * (X + 3);
+  return r + ((2 - r) & 3);
+}
+// one plane of the tile and the weights of its nine taps
+__host__ __device__ inline size_t halo_smem(int X, int ci, int nb) {
+  return (size_t)ci * 2 * halo_rows(X) + (size_t)9 * ci * nb * 2 + 128;
+}
+
+// Forward convolution and input gradient: a block owns 256 positions of a plane
+// x NB of the N output channels and takes the three input planes one after
+// another, each with its nine taps' weights in one buffer; the resident blocks
+// overlap their copies and MMAs.  The MMAs of an accumulator run over the taps
+// and, within a tap, over the 16-channel steps, the order of k_conv3d_tc: the
+// same sums bit for bit, so that no BF16 rounding downstream moves.  Waits and
+// errors as there.
+template <int NB>
+__global__ void __launch_bounds__(kHaloThreads) k_conv3d_halo(Shape s, const bf16 *__restrict__ X,
+                                                              const bf16 *__restrict__ W,
+                                                              float *__restrict__ Y, int Ci, int N,
+                                                              int tiles, int *err) {
+  constexpr int kCols = tc_cols(2 * NB);
+  extern __shared__ __align__(128) unsigned char halo_sm[];
+  __shared__ __align__(8) unsigned long long bar;
+  __shared__ unsigned tmem_base_s;
+  __shared__ int fail_s;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int XP = s.X + 2, PP = s.Y * XP, R = halo_rows(s.X);
+  const int pl = (int)blockIdx.x / tiles, p0 = ((int)blockIdx.x - pl * tiles) * kHaloM;
+  const int nmt = PP - p0 > 128 ? 2 : 1;  // MMA tiles with positions of the plane
+  const int used = nmt * 128 + 2 * (XP + 1);
+  const int z = pl % s.Z, n0 = (int)blockIdx.y * NB, groups = Ci / 8;
+  // [8-channel group][row], [tap][8-channel group][n]
+  unsigned char *A = halo_sm, *Bm = halo_sm + (size_t)16 * groups * R;
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     tc_smem_u32(&tmem_base_s)),
+                 "r"(kCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  if (t == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem_u32(&bar)));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fail_s = 0;
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const unsigned tmem = tmem_base_s;
+
+  const long long plane = (long long)s.Y * s.X;
+  bool ok = true;
+  for (int dz = 0; dz < 3; ++dz) {
+    if (dz) {  // the MMAs of the plane before have read the buffer
+      if (t == 0 && !tc_wait(&bar, (unsigned)((dz - 1) & 1))) fail_s = 1;
+      __syncthreads();
+      if (fail_s) {
+        ok = false;
+        break;
+      }
+    }
+    const bool in = z + dz - 1 >= 0 && z + dz - 1 < s.Z;
+    const bf16 *Xp = X + ((long long)pl + dz - 1) * plane * Ci;
+    for (int r = t >> 2; r < used; r += kHaloThreads / 4) {
+      const bf16 *src = in ? Xp + (long long)halo_voxel(s, p0, r) * Ci : X;
+      for (int g = t & 3; g < groups; g += 4)
+        tc_cp16(A + ((size_t)g * R + r) * 16, in ? src + g * 8 : X, in ? 16u : 0u);
+    }
+    for (int tap = 0; tap < 9; ++tap) {
+      const bf16 *src = W + ((long long)(dz * 9 + tap) * N + n0) * Ci;
+      unsigned char *dst = Bm + (size_t)tap * groups * NB * 16;
+      for (int n = t >> 2; n < NB; n += kHaloThreads / 4)
+        for (int g = t & 3; g < groups; g += 4)
+          tc_cp16(dst + (g * NB + n) * 16, src + (long long)n * Ci + g * 8, 16u);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (t == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned a0 = tc_desc_lo(tc_smem_u32(A), (unsigned)R);
+      unsigned b_lo = tc_desc_lo(tc_smem_u32(Bm), NB);
+      const unsigned hi = tc_desc_hi(8);
+#pragma unroll
+      for (int tap = 0; tap < 9; ++tap) {
+        unsigned a_lo = a0 + (unsigned)((XP + 1) + (tap / 3 - 1) * XP + (tap % 3 - 1));
+        for (int c = 0; c < groups; c += 2) {
+          tc_mma(tmem, a_lo, hi, b_lo, hi, tc_idesc(NB), (unsigned)(dz | tap | c));
+          if (nmt == 2)
+            tc_mma(tmem + NB, a_lo + 128, hi, b_lo, hi, tc_idesc(NB), (unsigned)(dz | tap | c));
+          a_lo += 2 * (unsigned)R;
+          b_lo += 2 * NB;
+        }
+      }
+      tc_commit(&bar);
+    }
+  }
+  if (ok) {
+    if (t == 0 && !tc_wait(&bar, 0)) fail_s = 1;  // the third phase
+    __syncthreads();
+    ok = !fail_s;
+  }
+  if (ok) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const int mt = warp >> 2, p = p0 + mt * 128 + (warp & 3) * 32 + lane;
+    const int y = p / XP, x = p - y * XP - 1;
+    const bool valid = p < PP && x >= 0 && x < s.X;
+    float *dst = Y + ((long long)pl * plane + (long long)y * s.X + x) * N + n0;
+    if (mt < nmt) {
+#pragma unroll
+      for (int c0 = 0; c0 < NB; c0 += 16) {
+        unsigned r[16];
+        tc_ld16(tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)(mt * NB + c0), r);
+        if (valid) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            reinterpret_cast<float4 *>(dst + c0)[q] =
+                make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
+                            __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+        }
+      }
+    }
+  } else if (t == 0) {
+    atomicExch(err, 1);
+    // (MMAs still in flight end within a bounded wait before the TMEM goes back)
+    tc_wait(&bar, 0);
+    tc_wait(&bar, 1);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
+  }
+}
+
+// Weight gradient: D[(dz, ci)][co] of the taps (dy, dx = -1, 0, 1) of one dy
+// accumulate in tensor memory over a range of voxels.  The three planes' groups
+// of 8 input channels are the rows of A, 128 at a time (grid.y: row block and
+// dy); K = 16 voxels per MMA, in two groups of 8 that lie in one row of the
+// plane each, so X must be a multiple of 8 and a plane of 16; both operands
+// MN-major.  A block walks the tiles of up to 128 voxels of its range, the
+// copies of the next tile running under the MMAs of this one, and adds its
+// sums to dW at the end.  Ranges, K groups and their order are those of
+// k_conv3d_wgrad_tc: the same partial sums bit for bit.
+constexpr int kWgM = 128;  // voxels of a tile
+
+// rows of its halo tile, = 2 (mod 4): the two rows and four channel groups that
+// 8 lanes copy together fall on different banks
+__host__ __device__ inline int wg_rows(int X) {
+  const int r = kWgM + 2 * (kWgM / X + 1) + 2;
+  return r + ((2 - r) & 3);
+}
+// buffers: the copies run up to three tiles ahead of the MMAs
+constexpr int wg_bufs(int co) { return co <= 48 ? 4 : 3; }
+template <int CO>
+size_t wg_smem(int X) {
+  return wg_bufs(CO) * ((size_t)16 * 16 * wg_rows(X) + (size_t)kWgM * CO * 2) + 128;
+}
+
+template <int CO>
+__global__ void __launch_bounds__(kHaloThreads)
+    k_conv3d_wgrad_halo(Shape s, const bf16 *__restrict__ dY, const bf16 *__restrict__ X,
+                        float *__restrict__ dW, int Ci, long long chunk, int *err) {
+  constexpr int kCols = tc_cols(3 * CO), G = CO / 8, NB = wg_bufs(CO);
+  extern __shared__ __align__(128) unsigned char halo_sm[];
+  __shared__ __align__(8) unsigned long long bar[NB];
+  __shared__ unsigned kdesc[NB][kWgM / 16];  // per K step: row of its first voxel, offset to the 8 others
+  __shared__ unsigned tmem_base_s;
+  __shared__ int fail_s;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int XP = s.X + 2, R = wg_rows(s.X), YX = s.Y * s.X;
+  const int mb = (int)blockIdx.y / 3, dy = (int)blockIdx.y % 3 - 1;
+  const long long M = s.voxels();
+  const int k0 = (int)(blockIdx.x * chunk), k1 = (int)(k0 + chunk < M ? k0 + chunk : M);
+  const int buf_bytes = 256 * R + kWgM * CO * 2;
+
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     tc_smem_u32(&tmem_base_s)),
+                 "r"(kCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  if (t == 0) {
+    for (int q = 0; q < NB; ++q)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem_u32(&bar[q])));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fail_s = 0;
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const unsigned tmem = tmem_base_s;
+
+  const int cg = Ci / 8;
+  // this thread copies the row groups 4 q + (t & 3) of the row block: their plane
+  // offset and channels (a group beyond the three planes stays zero)
+  int gz[4], gc[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int g = mb * 16 + 4 * q + (t & 3);
+    gz[q] = g / cg - 1;
+    gc[q] = (g - g / cg * cg) * 8;
+  }
+  // padded position of the voxel at offset v of a plane, less one: the row of the
+  // tile that its dx = -1 neighbour has
+  auto pos = [&](int v) { return v / s.X * XP + v % s.X; };
+  // voxels of the tile that starts at v: within a plane and the range
+  auto tile_len = [&](int v) { return min(min(kWgM, k1 - v), YX - v % YX); };
+  auto load = [&](int v, int len, int b) {
+    unsigned char *A = halo_sm + b * buf_bytes, *Bm = A + 256 * R;
+    const int pl = v / YX, off = v - pl * YX, z = pl % s.Z;
+    const int P0 = pos(off), used = pos(off + len - 1) + 3 - P0;
+    for (int r = t >> 2; r < used; r += kHaloThreads / 4) {
+      const int row = (P0 + r) / XP, px = P0 + r - row * XP - 1;
+      int y = row + dy, x = px < 0 ? s.X - 1 : (px >= s.X ? 0 : px);
+      y = y < 0 ? y + s.Y : (y >= s.Y ? y - s.Y : y);
+      const long long vox = (long long)pl * YX + y * s.X + x;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const bool in = gz[q] < 2 && z + gz[q] >= 0 && z + gz[q] < s.Z;
+        tc_cp16(A + ((4 * q + (t & 3)) * R + r) * 16,
+                in ? X + (vox + (long long)gz[q] * YX) * Ci + gc[q] : X, in ? 16u : 0u);
+      }
+    }
+    if (t < len / 16) {
+      const int p = pos(off + 16 * t);
+      kdesc[b][t] = (unsigned)(p - P0) | ((unsigned)(pos(off + 16 * t + 8) - p) << 16);
+    }
+    for (int e = t; e < len * G; e += kHaloThreads) {
+      const int r = e / G, g = e - r * G;
+      tc_cp16(Bm + (g * kWgM + r) * 16, dY + (long long)(v + r) * CO + g * 8, 16u);
+    }
+  };
+  // vl: the next tile to copy
+  int vl = k0, copied = 0;
+  auto copy_next = [&]() {
+    if (vl < k1) {
+      const int n = tile_len(vl);
+      load(vl, n, copied % NB);
+      vl += n;
+    }
+    ++copied;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int q = 0; q < NB - 1; ++q) copy_next();
+  int it = 0;
+  bool ok = true;
+  for (int v = k0; v < k1; ++it) {
+    const int len = tile_len(v), b = it % NB;
+    if (it) {  // the MMAs of the tile before have read the buffer that is copied to next
+      if (t == 0 && !tc_wait(&bar[(it - 1) % NB], (unsigned)(((it - 1) / NB) & 1))) fail_s = 1;
+      __syncthreads();
+      if (fail_s) {
+        ok = false;
+        break;
+      }
+    }
+    copy_next();
+    asm volatile("cp.async.wait_group %0;" ::"n"(NB - 1) : "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (t == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned a0 = tc_smem_u32(halo_sm + b * buf_bytes);
+      const unsigned a_base = tc_desc_lo(a0, 0), a_hi = tc_desc_hi((unsigned)R);
+      unsigned b_lo = tc_desc_lo(a0 + 256 * R, 8);
+      for (int k = 0; k < len / 16; ++k) {
+        const unsigned a_lo = a_base + kdesc[b][k];
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx)
+          tc_mma(tmem + dx * CO, a_lo + dx, a_hi, b_lo, tc_desc_hi(kWgM), tc_idesc_mn(CO),
+                 (unsigned)(it | k));
+        b_lo += 16;
+      }
+      tc_commit(&bar[b]);
+    }
+    v += len;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (ok) {  // the last commit covers every earlier tcgen05 operation
+    if (t == 0 && !tc_wait(&bar[(it - 1) % NB], (unsigned)(((it - 1) / NB) & 1))) fail_s = 1;
+    __syncthreads();
+    ok = !fail_s;
+  }
+  if (ok) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // row of D: channel ci of plane dz; the warps 0-3 and 4-7 take alternate columns
+    const int row = mb * 128 + (warp & 3) * 32 + lane, dz = row / Ci, ci = row - dz * Ci;
+    for (int c = (warp >> 2) * 16; c < 3 * CO; c += 32) {
+      unsigned r[16];
+      tc_ld16(tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c, r);
+      const int q = c / CO, co = c - q * CO, tap = dz * 9 + (dy + 1) * 3 + q;
+      if (dz < 3) {
+        float *dst = dW + ((long long)tap * CO + co) * Ci + ci;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) atomicAdd(dst + (long long)e * Ci, __uint_as_float(r[e]));
+      }
+    }
+  } else if (t == 0) {
+    atomicExch(err, 1);
+    for (int q = 0; q < 2 * NB; ++q) tc_wait(&bar[q % NB], q / NB);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
+  }
+}
+
 }  // namespace gen
 }  // namespace plc
