@@ -15,10 +15,14 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "plc_device.cuh"
+
 namespace plc {
 namespace gen {
 
 using bf16 = __nv_bfloat16;
+
+__device__ __forceinline__ float lrelu(float h) { return h > 0.f ? h : 0.2f * h; }
 
 struct Shape {
   int B, Z, Y, X;  // batch and spatial extents
@@ -106,6 +110,11 @@ __device__ __forceinline__ bool tc_wait(unsigned long long *bar, unsigned parity
 __device__ __forceinline__ void tc_cp16(void *dst, const void *src, unsigned src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tc_smem_u32(dst)), "l"(src),
                "r"(src_bytes)
+               : "memory");
+}
+
+__device__ __forceinline__ void tc_cp16s(unsigned dst, const void *src, unsigned src_bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes)
                : "memory");
 }
 
@@ -471,16 +480,22 @@ __global__ void __launch_bounds__(128) k_conv3d_wgrad_tc(Shape s, const bf16 *__
 // padding positions are computed and dropped (2 of X + 2).
 // ===========================================================================
 
+// divisions by the extents that the copies' index arithmetic needs
+struct HaloDiv {
+  FastDiv XP, X, YX;
+  explicit HaloDiv(const Shape &s) : XP(s.X + 2), X(s.X), YX(s.Y * s.X) {}
+};
+
 // Row q of a halo tile whose first output position is p0: its voxel within the
 // plane, periodic in y and x (rows that only padding outputs read map to some
 // voxel of the plane).
-__device__ __forceinline__ int halo_voxel(const Shape &s, int p0, int q) {
+__device__ __forceinline__ int halo_voxel(const Shape &s, const HaloDiv &d, int p0, int q) {
   const int XP = s.X + 2;
   const int pos = p0 - (XP + 1) + q + 2 * XP;  // not negative; two rows up
-  int y = pos / XP;
-  int x = pos - y * XP - 1;
-  y = (y - 2) % s.Y;
-  y = y < 0 ? y + s.Y : y;
+  const int row = d.XP.div(pos);
+  int x = pos - row * XP - 1, y = row - 2;
+  while (y < 0) y += s.Y;
+  while (y >= s.Y) y -= s.Y;
   x = x < 0 ? s.X - 1 : (x >= s.X ? 0 : x);
   return y * s.X + x;
 }
@@ -535,8 +550,20 @@ __host__ __device__ inline int halo_rows(int X) {
 }
 // one plane of the tile and the weights of its nine taps
 __host__ __device__ inline size_t halo_smem(int X, int ci, int nb) {
-  return (size_t)ci * 2 * halo_rows(X) + (size_t)9 * ci * nb * 2 + 128;
+  return (size_t)(ci * 2 + 4) * halo_rows(X) + (size_t)9 * ci * nb * 2 + 128;
 }
+
+// What the epilogue of a convolution does with its FP32 sums: stores them (pre,
+// if not null) and, with film, h = gamma * sum + beta, gamma = 1 + A0 + A1 r and
+// beta = B0 + B1 r per sample, plane and channel, as BF16 lrelu(h) (act) or FP32 h
+// (out).
+struct ConvOut {
+  float *pre = nullptr;
+  const float *film = nullptr;  // A0, A1, B0, B1 [z][c]
+  const float *r = nullptr;     // [b]
+  bf16 *act = nullptr;
+  float *out = nullptr;
+};
 
 // Forward convolution and input gradient: a block owns 256 positions of a plane
 // x NB of the N output channels and takes the three input planes one after
@@ -548,9 +575,10 @@ __host__ __device__ inline size_t halo_smem(int X, int ci, int nb) {
 template <int NB>
 __global__ void __launch_bounds__(kHaloThreads) k_conv3d_halo(Shape s, const bf16 *__restrict__ X,
                                                               const bf16 *__restrict__ W,
-                                                              float *__restrict__ Y, int Ci, int N,
-                                                              int tiles, int *err) {
+                                                              ConvOut o, int Ci, int N, int tiles,
+                                                              HaloDiv d, int *err) {
   constexpr int kCols = tc_cols(2 * NB);
+  __shared__ float gam[NB], bet[NB];
   extern __shared__ __align__(128) unsigned char halo_sm[];
   __shared__ __align__(8) unsigned long long bar;
   __shared__ unsigned tmem_base_s;
@@ -561,8 +589,16 @@ __global__ void __launch_bounds__(kHaloThreads) k_conv3d_halo(Shape s, const bf1
   const int nmt = PP - p0 > 128 ? 2 : 1;  // MMA tiles with positions of the plane
   const int used = nmt * 128 + 2 * (XP + 1);
   const int z = pl % s.Z, n0 = (int)blockIdx.y * NB, groups = Ci / 8;
-  // [8-channel group][row], [tap][8-channel group][n]
+  // [8-channel group][row], [tap][8-channel group][n], the rows' elements in a plane
   unsigned char *A = halo_sm, *Bm = halo_sm + (size_t)16 * groups * R;
+  int *src_row = reinterpret_cast<int *>(Bm + (size_t)9 * groups * NB * 16);
+  for (int r = t; r < used; r += kHaloThreads) src_row[r] = halo_voxel(s, d, p0, r) * Ci;
+  if (o.film && t < NB) {
+    const long long zc = (long long)s.Z * N, q = (long long)z * N + n0 + t;
+    const float rb = o.r[pl / s.Z];
+    gam[t] = 1.f + o.film[q] + o.film[zc + q] * rb;
+    bet[t] = o.film[2 * zc + q] + o.film[3 * zc + q] * rb;
+  }
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -593,17 +629,27 @@ __global__ void __launch_bounds__(kHaloThreads) k_conv3d_halo(Shape s, const bf1
     }
     const bool in = z + dz - 1 >= 0 && z + dz - 1 < s.Z;
     const bf16 *Xp = X + ((long long)pl + dz - 1) * plane * Ci;
+    const int g0 = t & 3;
     for (int r = t >> 2; r < used; r += kHaloThreads / 4) {
-      const bf16 *src = in ? Xp + (long long)halo_voxel(s, p0, r) * Ci : X;
-      for (int g = t & 3; g < groups; g += 4)
-        tc_cp16(A + ((size_t)g * R + r) * 16, in ? src + g * 8 : X, in ? 16u : 0u);
+      const bf16 *src = in ? Xp + src_row[r] + g0 * 8 : X;
+      unsigned dst = tc_smem_u32(A) + (unsigned)(g0 * R + r) * 16u;
+      for (int g = g0; g < groups; g += 4) {
+        tc_cp16s(dst, src, in ? 16u : 0u);
+        src += in ? 32 : 0;
+        dst += 64u * (unsigned)R;
+      }
     }
-    for (int tap = 0; tap < 9; ++tap) {
-      const bf16 *src = W + ((long long)(dz * 9 + tap) * N + n0) * Ci;
-      unsigned char *dst = Bm + (size_t)tap * groups * NB * 16;
-      for (int n = t >> 2; n < NB; n += kHaloThreads / 4)
-        for (int g = t & 3; g < groups; g += 4)
-          tc_cp16(dst + (g * NB + n) * 16, src + (long long)n * Ci + g * 8, 16u);
+    // rows tap * NB + n of the weights
+    const bf16 *Wp = W + ((long long)dz * 9 * N + n0) * Ci + g0 * 8;
+    for (int rr = t >> 2; rr < 9 * NB; rr += kHaloThreads / 4) {
+      const int tap = rr / NB, n = rr - tap * NB;
+      const bf16 *src = Wp + (tap * N + n) * Ci;
+      unsigned dst = tc_smem_u32(Bm) + (unsigned)((tap * groups + g0) * NB + n) * 16u;
+      for (int g = g0; g < groups; g += 4) {
+        tc_cp16s(dst, src, 16u);
+        src += 32;
+        dst += 64u * NB;
+      }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -638,18 +684,37 @@ __global__ void __launch_bounds__(kHaloThreads) k_conv3d_halo(Shape s, const bf1
     const int mt = warp >> 2, p = p0 + mt * 128 + (warp & 3) * 32 + lane;
     const int y = p / XP, x = p - y * XP - 1;
     const bool valid = p < PP && x >= 0 && x < s.X;
-    float *dst = Y + ((long long)pl * plane + (long long)y * s.X + x) * N + n0;
+    const long long at = ((long long)pl * plane + (long long)y * s.X + x) * N + n0;
     if (mt < nmt) {
 #pragma unroll
       for (int c0 = 0; c0 < NB; c0 += 16) {
         unsigned r[16];
         tc_ld16(tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)(mt * NB + c0), r);
-        if (valid) {
+        if (!valid) continue;
+        if (o.pre) {
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            reinterpret_cast<float4 *>(dst + c0)[q] =
+            reinterpret_cast<float4 *>(o.pre + at + c0)[q] =
                 make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
                             __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+        }
+        if (!o.film) continue;
+        float h[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) h[q] = gam[c0 + q] * __uint_as_float(r[q]) + bet[c0 + q];
+        if (o.act) {
+          __align__(16) __nv_bfloat162 a[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            a[q] = __floats2bfloat162_rn(lrelu(h[2 * q]), lrelu(h[2 * q + 1]));
+          uint4 *dst = reinterpret_cast<uint4 *>(o.act + at + c0);
+          dst[0] = reinterpret_cast<const uint4 *>(a)[0];
+          dst[1] = reinterpret_cast<const uint4 *>(a)[1];
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            reinterpret_cast<float4 *>(o.out + at + c0)[q] =
+                make_float4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
         }
       }
     }
@@ -684,7 +749,7 @@ __host__ __device__ inline int wg_rows(int X) {
   const int r = kWgM + 2 * (kWgM / X + 1) + 2;
   return r + ((2 - r) & 3);
 }
-// buffers: the copies run up to three tiles ahead of the MMAs
+// buffers: the copies run one or two tiles ahead of the MMAs, which have as long to finish
 constexpr int wg_bufs(int co) { return co <= 48 ? 4 : 3; }
 template <int CO>
 size_t wg_smem(int X) {
@@ -694,7 +759,7 @@ size_t wg_smem(int X) {
 template <int CO>
 __global__ void __launch_bounds__(kHaloThreads)
     k_conv3d_wgrad_halo(Shape s, const bf16 *__restrict__ dY, const bf16 *__restrict__ X,
-                        float *__restrict__ dW, int Ci, long long chunk, int *err) {
+                        float *__restrict__ dW, int Ci, long long chunk, HaloDiv d, int *err) {
   constexpr int kCols = tc_cols(3 * CO), G = CO / 8, NB = wg_bufs(CO);
   extern __shared__ __align__(128) unsigned char halo_sm[];
   __shared__ __align__(8) unsigned long long bar[NB];
@@ -737,15 +802,15 @@ __global__ void __launch_bounds__(kHaloThreads)
   }
   // padded position of the voxel at offset v of a plane, less one: the row of the
   // tile that its dx = -1 neighbour has
-  auto pos = [&](int v) { return v / s.X * XP + v % s.X; };
+  auto pos = [&](int v) { return v + 2 * d.X.div(v); };
   // voxels of the tile that starts at v: within a plane and the range
-  auto tile_len = [&](int v) { return min(min(kWgM, k1 - v), YX - v % YX); };
+  auto tile_len = [&](int v) { return min(min(kWgM, k1 - v), YX - (v - d.YX.div(v) * YX)); };
   auto load = [&](int v, int len, int b) {
     unsigned char *A = halo_sm + b * buf_bytes, *Bm = A + 256 * R;
-    const int pl = v / YX, off = v - pl * YX, z = pl % s.Z;
+    const int pl = d.YX.div(v), off = v - pl * YX, z = pl % s.Z;
     const int P0 = pos(off), used = pos(off + len - 1) + 3 - P0;
     for (int r = t >> 2; r < used; r += kHaloThreads / 4) {
-      const int row = (P0 + r) / XP, px = P0 + r - row * XP - 1;
+      const int row = d.XP.div(P0 + r), px = P0 + r - row * XP - 1;
       int y = row + dy, x = px < 0 ? s.X - 1 : (px >= s.X ? 0 : px);
       y = y < 0 ? y + s.Y : (y >= s.Y ? y - s.Y : y);
       const long long vox = (long long)pl * YX + y * s.X + x;
@@ -762,7 +827,7 @@ __global__ void __launch_bounds__(kHaloThreads)
     }
     for (int e = t; e < len * G; e += kHaloThreads) {
       const int r = e / G, g = e - r * G;
-      tc_cp16(Bm + (g * kWgM + r) * 16, dY + (long long)(v + r) * CO + g * 8, 16u);
+      tc_cp16(Bm + (g * kWgM + r) * 16, dY + ((long long)v * CO + e * 8), 16u);
     }
   };
   // vl: the next tile to copy
@@ -776,13 +841,13 @@ __global__ void __launch_bounds__(kHaloThreads)
     ++copied;
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  for (int q = 0; q < NB - 1; ++q) copy_next();
+  for (int q = 0; q < NB - 2; ++q) copy_next();
   int it = 0;
   bool ok = true;
   for (int v = k0; v < k1; ++it) {
     const int len = tile_len(v), b = it % NB;
-    if (it) {  // the MMAs of the tile before have read the buffer that is copied to next
-      if (t == 0 && !tc_wait(&bar[(it - 1) % NB], (unsigned)(((it - 1) / NB) & 1))) fail_s = 1;
+    if (it >= 2) {  // the MMAs of two tiles before have read the buffer that is copied to next
+      if (t == 0 && !tc_wait(&bar[(it - 2) % NB], (unsigned)(((it - 2) / NB) & 1))) fail_s = 1;
       __syncthreads();
       if (fail_s) {
         ok = false;
@@ -790,7 +855,7 @@ __global__ void __launch_bounds__(kHaloThreads)
       }
     }
     copy_next();
-    asm volatile("cp.async.wait_group %0;" ::"n"(NB - 1) : "memory");
+    asm volatile("cp.async.wait_group %0;" ::"n"(NB - 2) : "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (t == 0) {
