@@ -696,7 +696,7 @@ bool wgrad_halo(plc_gen *gn, Shape s, const bf16 *dy, const bf16 *x, float *dw, 
   if (s.X % 8 || (s.Y * s.X) % 16 || smem > kSmemMax) return false;
   const WgradSplit w(s.voxels());
   k_conv3d_wgrad_halo<CO><<<dim3((unsigned)w.splits, (unsigned)((3 * ci + 127) / 128 * 3)),
-                            kHaloThreads, smem, gn->stream>>>(s, dy, x, dw, ci, w.chunk, HaloDiv(s),
+                            kHaloThreads + 32, smem, gn->stream>>>(s, dy, x, dw, ci, w.chunk, HaloDiv(s),
                                                               gn->derr);
   *e = cudaGetLastError();
   return true;

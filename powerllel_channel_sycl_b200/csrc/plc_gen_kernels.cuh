@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(128) k_conv3d_wgrad_tc(Shape s, const bf16 *__
 //
 // The kernels above copy the im2col rows of every tap, 27 reads of each input
 // value from L2, which is what bounded them (64 -> 32 channels on 4 x 64 x 48 x 64
-// voxels: 0.91 ms forward, 2.07 ms weight gradient; here 0.39 and 0.83).  Here a plane (b, z) is
+// voxels: 0.91 ms forward, 2.07 ms weight gradient; here 0.34 and 0.49).  Here a plane (b, z) is
 // numbered by padded positions p = y * (X + 2) + x + 1: the neighbour at (dz,
 // dy, dx) of the output at p is the input at p + dy * (X + 2) + dx of plane
 // z + dz, for every p whose x is not one of the two padding columns.  A tile of
@@ -749,7 +749,7 @@ __host__ __device__ inline int wg_rows(int X) {
   const int r = kWgM + 2 * (kWgM / X + 1) + 2;
   return r + ((2 - r) & 3);
 }
-// buffers: the copies run one or two tiles ahead of the MMAs, which have as long to finish
+// buffers
 constexpr int wg_bufs(int co) { return co <= 48 ? 4 : 3; }
 template <int CO>
 size_t wg_smem(int X) {
@@ -757,12 +757,12 @@ size_t wg_smem(int X) {
 }
 
 template <int CO>
-__global__ void __launch_bounds__(kHaloThreads)
+__global__ void __launch_bounds__(kHaloThreads + 32)
     k_conv3d_wgrad_halo(Shape s, const bf16 *__restrict__ dY, const bf16 *__restrict__ X,
                         float *__restrict__ dW, int Ci, long long chunk, HaloDiv d, int *err) {
   constexpr int kCols = tc_cols(3 * CO), G = CO / 8, NB = wg_bufs(CO);
   extern __shared__ __align__(128) unsigned char halo_sm[];
-  __shared__ __align__(8) unsigned long long bar[NB];
+  __shared__ __align__(8) unsigned long long full[NB], empty[NB];
   __shared__ unsigned kdesc[NB][kWgM / 16];  // per K step: row of its first voxel, offset to the 8 others
   __shared__ unsigned tmem_base_s;
   __shared__ int fail_s;
@@ -780,8 +780,11 @@ __global__ void __launch_bounds__(kHaloThreads)
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
   if (t == 0) {
-    for (int q = 0; q < NB; ++q)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem_u32(&bar[q])));
+    for (int q = 0; q < NB; ++q) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem_u32(&full[q])),
+                   "r"(kHaloThreads));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem_u32(&empty[q])));
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fail_s = 0;
   }
@@ -830,62 +833,68 @@ __global__ void __launch_bounds__(kHaloThreads)
       tc_cp16(Bm + (g * kWgM + r) * 16, dY + ((long long)v * CO + e * 8), 16u);
     }
   };
-  // vl: the next tile to copy
-  int vl = k0, copied = 0;
-  auto copy_next = [&]() {
-    if (vl < k1) {
-      const int n = tile_len(vl);
-      load(vl, n, copied % NB);
-      vl += n;
-    }
-    ++copied;
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  for (int q = 0; q < NB - 2; ++q) copy_next();
-  int it = 0;
+  // The copying warps run ahead of the MMA warp by up to NB tiles: full[b] is
+  // reached when every copying thread's part of the tile in buffer b has
+  // landed, empty[b] when the MMAs have read it.  (One set of threads copying
+  // and issuing in turn took 2.6 us a tile of 32 x 32 channels against 1.75.)
   bool ok = true;
-  for (int v = k0; v < k1; ++it) {
-    const int len = tile_len(v), b = it % NB;
-    if (it >= 2) {  // the MMAs of two tiles before have read the buffer that is copied to next
-      if (t == 0 && !tc_wait(&bar[(it - 2) % NB], (unsigned)(((it - 2) / NB) & 1))) fail_s = 1;
-      __syncthreads();
-      if (fail_s) {
-        ok = false;
-        break;
+  int tiles = 0;
+  if (warp < kHaloThreads / 32) {
+    constexpr int D = NB - 2;  // tiles in flight behind the newest
+    auto landed = [&](int i) {  // tile i is this thread's oldest in flight
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc_smem_u32(&full[i % NB]))
+                   : "memory");
+    };
+    for (int v = k0; v < k1 && ok; ++tiles) {
+      const int len = tile_len(v), b = tiles % NB;
+      if (tiles >= NB) ok = tc_wait(&empty[b], (unsigned)((tiles / NB - 1) & 1));
+      if (ok) {
+        load(v, len, b);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (tiles >= D) {
+          asm volatile("cp.async.wait_group %0;" ::"n"(D) : "memory");
+          landed(tiles - D);
+        }
       }
+      v += len;
     }
-    copy_next();
-    asm volatile("cp.async.wait_group %0;" ::"n"(NB - 2) : "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (t == 0) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (ok) {
+      for (int i = max(0, tiles - D); i < tiles; ++i) landed(i);
+      // the last commit covers every earlier tcgen05 operation
+      ok = tc_wait(&empty[(tiles - 1) % NB], (unsigned)(((tiles - 1) / NB) & 1));
+    }
+  } else if (lane == 0) {
+    const unsigned a_hi = tc_desc_hi((unsigned)R);
+    for (int v = k0; v < k1; ++tiles) {
+      const int len = tile_len(v), b = tiles % NB;
+      ok = tc_wait(&full[b], (unsigned)((tiles / NB) & 1));
+      if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const unsigned a0 = tc_smem_u32(halo_sm + b * buf_bytes);
-      const unsigned a_base = tc_desc_lo(a0, 0), a_hi = tc_desc_hi((unsigned)R);
+      const unsigned a_base = tc_desc_lo(a0, 0);
       unsigned b_lo = tc_desc_lo(a0 + 256 * R, 8);
       for (int k = 0; k < len / 16; ++k) {
         const unsigned a_lo = a_base + kdesc[b][k];
 #pragma unroll
         for (int dx = 0; dx < 3; ++dx)
           tc_mma(tmem + dx * CO, a_lo + dx, a_hi, b_lo, tc_desc_hi(kWgM), tc_idesc_mn(CO),
-                 (unsigned)(it | k));
+                 (unsigned)(tiles | k));
         b_lo += 16;
       }
-      tc_commit(&bar[b]);
+      tc_commit(&empty[b]);
+      v += len;
     }
-    v += len;
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  if (ok) {  // the last commit covers every earlier tcgen05 operation
-    if (t == 0 && !tc_wait(&bar[(it - 1) % NB], (unsigned)(((it - 1) / NB) & 1))) fail_s = 1;
-    __syncthreads();
-    ok = !fail_s;
-  }
+  if (!ok) fail_s = 1;
+  __syncthreads();
+  ok = !fail_s;
   if (ok) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // row of D: channel ci of plane dz; the warps 0-3 and 4-7 take alternate columns
     const int row = mb * 128 + (warp & 3) * 32 + lane, dz = row / Ci, ci = row - dz * Ci;
-    for (int c = (warp >> 2) * 16; c < 3 * CO; c += 32) {
+    for (int c = warp < 8 ? (warp >> 2) * 16 : 3 * CO; c < 3 * CO; c += 32) {
       unsigned r[16];
       tc_ld16(tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)c, r);
       const int q = c / CO, co = c - q * CO, tap = dz * 9 + (dy + 1) * 3 + q;
@@ -897,7 +906,7 @@ __global__ void __launch_bounds__(kHaloThreads)
     }
   } else if (t == 0) {
     atomicExch(err, 1);
-    for (int q = 0; q < 2 * NB; ++q) tc_wait(&bar[q % NB], q / NB);
+    for (int q = 0; q < 2 * NB; ++q) tc_wait(&empty[q % NB], q / NB);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
