@@ -64,19 +64,17 @@ WORKLOADS = {
 # counted once (halos and 1-D coefficients excluded).
 KERNEL_BYTES_PER_POINT = {
     "rk1+bound(u1)": 48,          # read u,v,w; write u1,v1,w1
-    "rk2+bound(u)": 72,           # read u1,v1,w1,u,v,w; write u,v,w
+    "rk2+bound(u)+mean": 72,      # read u1,v1,w1,u,v,w; write u,v,w
     "calcRHS+fft_x_fwd": 32,      # read u,v,w; write spectral array
     "fft_y_fwd": 16,              # spectral array in place
     "trid_z": 16,                 # spectral array in place (pivot table excluded)
     "fft_y_bwd": 16,
     "fft_x_bwd+bound(p)": 16,     # read spectral array; write p
-    "correct+mean": 56,           # read p,u,v,w; write u,v,w
-    "force+bound(u)": 16,         # read u; write u
+    "correct+force+bound(u)": 56,  # read p,u,v,w; write u,v,w
 }
-STEP_BYTES_PER_POINT = sum(KERNEL_BYTES_PER_POINT.values())  # 288
+STEP_BYTES_PER_POINT = sum(KERNEL_BYTES_PER_POINT.values())  # 272
 # the mixed form stores every field in FP32 (half the bytes; the pivot table
-# excluded, as above); its RK2 also sums the bulk mean and its correction
-# applies the forcing, so it has no separate forcing pass
+# excluded, as above)
 MIXED_BYTES_PER_POINT = {
     "rk1+bound(u1)": 24,          # read u,v,w; write u1,v1,w1
     "rk2+bound(u)+mean": 36,      # read u1,v1,w1,u,v,w; write u,v,w

@@ -324,12 +324,14 @@ const char *const kStepKernelNames[] = {
     "rk1+bound(u1)", "rk2+bound(u)", "calcRHS+fft_x_fwd", "fft_y_fwd", "trid_z",
     "fft_y_bwd",     "fft_x_bwd+bound(p)", "correct+mean", "force+bound(u)"};
 constexpr int kStepKernels = 9;
-// the mixed form sums the bulk mean in RK2 and forces in the correction
-const char *const kStepKernelNamesMixed[] = {
+// the mixed form, and the FP64 form of a channel forced in x alone, take the bulk
+// mean after RK2 and force in the correction
+const char *const kStepKernelNamesForced[] = {
     "rk1+bound(u1)", "rk2+bound(u)+mean", "calcRHS+fft_x_fwd", "fft_y_fwd", "trid_z",
     "fft_y_bwd",     "fft_x_bwd+bound(p)", "correct+force+bound(u)"};
-constexpr int kStepKernelsMixed = 8;  // the one-block bulk_force sum is timed with RK2
-int step_kernels(const plc_ctx *c) { return c->mixed ? kStepKernelsMixed : kStepKernels; }
+constexpr int kStepKernelsForced = 8;  // the mean is timed with RK2
+bool step_forced(const plc_ctx *c) { return c->mixed || forced_early(c); }
+int step_kernels(const plc_ctx *c) { return step_forced(c) ? kStepKernelsForced : kStepKernels; }
 
 // Launches of one fused step (main.cc:116-154) on the context's fields, in
 // the context's storage type T.  With ev != nullptr, ev[0] is recorded before
@@ -349,6 +351,8 @@ int enqueue_step_t(plc_ctx *c, T *const *f, cudaStream_t s, cudaEvent_t *ev) {
   PLC_CUDA(c, launch_rk(c, 1, true, u_crf, u, v, w, u1, v1, w1, s));     // RK1 + bound(u1)
   PLC_CUDA(c, mark());
   PLC_CUDA(c, launch_rk(c, 2, true, u_crf, u1, v1, w1, u, v, w, s));     // RK2 + bound(u)
+  if constexpr (std::is_same<T, double>::value)
+    if (forced_early(c)) PLC_CUDA(c, launch_mean_force(c, u, s));
   PLC_CUDA(c, mark());
   if constexpr (std::is_same<T, double>::value)
     PLC_CUDA(c, launch_fft_x_fwd(c, nullptr, u, v, w, spec, s));         // calcRHS + x-FFT
@@ -366,8 +370,10 @@ int enqueue_step_t(plc_ctx *c, T *const *f, cudaStream_t s, cudaEvent_t *ev) {
   PLC_CUDA(c, launch_correct(c, true, p, u, v, w, s));                   // correct + mean
   PLC_CUDA(c, mark());
   if constexpr (std::is_same<T, double>::value) {
-    PLC_CUDA(c, launch_force_apply(c, true, u, v, w, s));                // force + bound(u)
-    PLC_CUDA(c, mark());
+    if (!forced_early(c)) {
+      PLC_CUDA(c, launch_force_apply(c, true, u, v, w, s));              // force + bound(u)
+      PLC_CUDA(c, mark());
+    }
   }
   return PLC_OK;
 }
@@ -1567,8 +1573,8 @@ const char *plc_step_kernel_name(int i) {
 }
 
 const char *plc_step_kernel_name_ctx(const plc_ctx *c, int i) {
-  if (!c || !c->mixed) return plc_step_kernel_name(i);
-  return (i >= 0 && i < kStepKernelsMixed) ? kStepKernelNamesMixed[i] : "";
+  if (!c || !step_forced(c)) return plc_step_kernel_name(i);
+  return (i >= 0 && i < kStepKernelsForced) ? kStepKernelNamesForced[i] : "";
 }
 
 int plc_mesh_by_func(int mesh_type, int stretch_func, double stretch_ratio, int nz, double lz,

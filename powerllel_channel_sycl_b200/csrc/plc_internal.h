@@ -276,6 +276,7 @@ cudaError_t launch_init_flow(const plc_ctx *c, double *u, double *v, double *w,
                              const double *d_prof, cudaStream_t s);
 cudaError_t launch_init_flow(const plc_ctx *c, float *u, float *v, float *w,
                              const double *d_prof, cudaStream_t s);
+cudaError_t launch_mean_force(const plc_ctx *c, const double *u, cudaStream_t s);
 cudaError_t launch_scale(const plc_ctx *c, double *var, const double *d_mult,
                          cudaStream_t s);
 cudaError_t launch_scale(const plc_ctx *c, float *var, const double *d_mult,
@@ -414,6 +415,12 @@ inline int rk_chunk(const plc_ctx *c, int kmax) {
   if (k > kmax) k = kmax;
   k /= c->rk_cut;
   return k < c->nz ? k : c->nz;
+}
+// FP64 form: the bulk mean is taken before the correction, which applies the force
+// (channels forced in x alone; the mean of w changes with the correction, so
+// others keep the passes after it)
+inline bool forced_early(const plc_ctx *c) {
+  return !c->mixed && c->prm.is_forced[0] && !c->prm.is_forced[1] && !c->prm.is_forced[2];
 }
 // whether the 8-plane blocks of the RK stages leave the device less than two
 // waves of its resident blocks

@@ -774,6 +774,52 @@ __global__ void __launch_bounds__(256) k_mean(Geo g, StepConst *sc, int comp, in
   }
 }
 
+// The forcing of a channel forced in x alone, before the correction:
+// sc->mean[0] = Mean(u), sc->force[0] = vel_force - mean[0]
+// (mod_calcVel.cc:280-301).  The correction changes each x-line of u by -dt/dx
+// times sum_i (p(i+1) - p(i)), zero on the periodic line, so the mean of the field
+// that the second RK stage leaves is that of the corrected field up to the
+// rounding of each point, and the correction can add the force: one read of u
+// here (8 B/pt) for its read and write in a pass of its own and the sums in the
+// correction.  Summed inside RK2 instead, the FP64 pipe that bounds that stage
+// took 0.20 ms more at 768 x 384 x 256; this pass takes 0.15.
+// A warp takes four rows at a time, so that short rows keep as many loads in
+// flight.
+__global__ void __launch_bounds__(256) k_mean_force(Geo g, StepConst *sc, double vel_force,
+                                                    const double *__restrict__ u,
+                                                    double *partials, unsigned int *counter) {
+  __shared__ double smem[2 * 32];
+  DD s[1] = {{0.0, 0.0}};
+  const int nrows = g.ny * g.nz, lane = threadIdx.x & 31;
+  const int warps = (int)(gridDim.x * blockDim.x) >> 5;
+  for (int r0 = 4 * (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); r0 < nrows;
+       r0 += 4 * warps) {
+    const double *p[4];
+    double wz[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int row = min(r0 + q, nrows - 1), k = row / g.ny + 1, j = row - (k - 1) * g.ny + 1;
+      p[q] = u + g.at(1, j, k);
+      wz[q] = r0 + q < nrows ? __ldg(g.dzflzi + k) : 0.0;
+    }
+#pragma unroll 2
+    for (int i = lane; i < g.nx; i += 32) {
+      double x[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) x[q] = p[q][i];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) dd_add(s[0], x[q] * wz[q]);
+    }
+  }
+  block_sum<1>(s, smem);
+  if (grid_sum_last<1>(s, partials, counter, gridDim.x, blockIdx.x, smem)) {
+    const double mean = (s[0].hi + s[0].lo) / g.nx / g.ny;
+    sc->mean[0] = mean;
+    sc->force[0] = vel_force - mean;
+    sc->mean[1] = sc->mean[2] = sc->force[1] = sc->force[2] = 0.0;
+  }
+}
+
 // correctVel (mod_calcVel.cc:253-278), interior only.  T = float: the
 // mixed form's plain correction (the projection of plc_project).
 template <class T>
@@ -898,9 +944,9 @@ __global__ void __launch_bounds__(256, 2) k_correct_fused(Geo g, StepConst *sc, 
   }
 }
 
-// The mixed form's fused correction: correctVel (mod_calcVel.cc:272-274) plus
-// the forcing sc->force[d] that its fused RK2 stage has already reduced
-// (0 for unforced components), written with the halo images and wall ghosts.
+// The fused correction of the mixed form, and of the FP64 form where it is forced
+// in x alone (correction and forcing 0.90 + 0.21 -> 0.67 ms there): correctVel (mod_calcVel.cc:272-274) plus the forcing sc->force[d]
+// that has already been reduced (0 for unforced components), written with the halo images and wall ghosts.
 // No reduction, so a plain grid: each thread takes KZ planes of one column
 // (p(k+1) of a plane is p(k) of the next) with all loads issued first.
 template <class T, int KZ>
@@ -1522,24 +1568,17 @@ cudaError_t launch_rk_tma(const plc_ctx *c, const CUtensorMap &mu, const CUtenso
                                                     ow, kchunk, c->d_err,
                                                     STAGE == 2 ? c->order[SK_RK2] : 0);
   };
-  // without the halo writes the two kernels are the same
-  const bool inl = FUSE && (STAGE == 1 || rk_small_grid(c));
   const std::true_type yes{};
   const std::false_type no{};
-  if constexpr (FUSE) {
-    if (inl) {
-      if (u_crf != 0.0)
-        go(yes, yes);
-      else
-        go(no, yes);
-      return cudaGetLastError();
-    }
-  }
-  if constexpr (!FUSE || STAGE == 2) {
-    if (u_crf != 0.0)
-      go(yes, no);
-    else
-      go(no, no);
+  const bool crf = u_crf != 0.0;
+  if constexpr (!FUSE) {  // without the halo writes the two kernels are the same
+    crf ? go(yes, no) : go(no, no);
+  } else if constexpr (STAGE == 1) {
+    crf ? go(yes, yes) : go(no, yes);
+  } else if (rk_small_grid(c)) {
+    crf ? go(yes, yes) : go(no, yes);
+  } else {
+    crf ? go(yes, no) : go(no, no);
   }
   return cudaGetLastError();
 }
@@ -1609,27 +1648,31 @@ namespace {
 // 0.437 for 4, FP32, 768x384x256)
 constexpr int kCorrKzMixed = 8;
 
+// FP64: 4 planes (their loads live in registers)
+constexpr int kCorrKz64 = 4;
+
 template <class T>
 cudaError_t correct_fused_t(const plc_ctx *c, const T *p, T *u, T *v, T *w, cudaStream_t s) {
-  // KZ planes per work item (the loads of one item live in registers): 6 in
-  // FP32, 4 in FP64; 2 resident blocks per SM (launch bounds)
-  constexpr int KZ = sizeof(T) == 4 ? 6 : 4;
-  constexpr int kBlocksPerSm = 2;
-  // one wave of resident blocks, at most the items
-  const long long items =
-      (long long)((c->nx + 31) / 32) * ((c->ny + 7) / 8) * ((c->nz + KZ - 1) / KZ);
-  long long nb = (long long)kBlocksPerSm * c->num_sms;
-  if (nb > items) nb = items;
-  if (nb > kMaxBlocksReduce) nb = kMaxBlocksReduce;
-  if (c->mixed) {
-    // the mixed form's fused RK2 stage has reduced the forcing already
-    constexpr int KZF = kCorrKzMixed;
-    dim3 grid((c->nx + BX - 1) / BX, (c->ny + BY - 1) / BY, (c->nz + KZF - 1) / KZF);
-    k_correct_forced<T, KZF><<<grid, dim3(BX, BY), 0, s>>>(c->geo(), c->d_sc, c->prm.u_crf, p, u,
-                                                          v, w);
-  } else {
+  if (c->mixed || forced_early(c)) {
+    // the forcing has been reduced from the field that RK2 left
+    constexpr int KZ = sizeof(T) == 4 ? kCorrKzMixed : kCorrKz64;
+    dim3 grid((c->nx + BX - 1) / BX, (c->ny + BY - 1) / BY, (c->nz + KZ - 1) / KZ);
+    k_correct_forced<T, KZ><<<grid, dim3(BX, BY), 0, s>>>(c->geo(), c->d_sc, c->prm.u_crf, p, u, v,
+                                                         w);
+    return cudaGetLastError();
+  }
+  if constexpr (sizeof(T) == 8) {
+    // KZ planes per work item; 2 resident blocks per SM (launch bounds)
+    constexpr int KZ = 4;
+    constexpr int kBlocksPerSm = 2;
+    // one wave of resident blocks, at most the items
+    const long long items =
+        (long long)((c->nx + 31) / 32) * ((c->ny + 7) / 8) * ((c->nz + KZ - 1) / KZ);
+    long long nb = (long long)kBlocksPerSm * c->num_sms;
+    if (nb > items) nb = items;
+    if (nb > kMaxBlocksReduce) nb = kMaxBlocksReduce;
     k_correct_fused<T, KZ><<<(unsigned)nb, 256, 0, s>>>(c->geo(), c->d_sc, force_cfg(c), p, u, v,
-                                                         w, c->d_partials, c->d_counter);
+                                                       w, c->d_partials, c->d_counter);
   }
   return cudaGetLastError();
 }
@@ -1691,6 +1734,14 @@ cudaError_t launch_mean(const plc_ctx *c, int comp, int nxg, int nyg, const floa
                         cudaStream_t s) {
   k_mean<float><<<reduce_blocks(c), 256, 0, s>>>(c->geo(), c->d_sc, comp, nxg, nyg, var,
                                                  c->d_partials, c->d_counter + 1);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mean_force(const plc_ctx *c, const double *u, cudaStream_t s) {
+  const long long rows = (long long)c->ny * c->nz;
+  const int nb = (int)std::min<long long>((rows + 31) / 32, 8ll * c->device_sms);
+  k_mean_force<<<nb, 256, 0, s>>>(c->geo(), c->d_sc, c->prm.vel_force[0], u, c->d_partials,
+                                  c->d_counter);
   return cudaGetLastError();
 }
 
