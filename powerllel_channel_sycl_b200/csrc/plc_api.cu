@@ -280,7 +280,8 @@ cudaError_t rk_autotune(plc_ctx *c) {
   std::vector<std::pair<int, int>> candidates;  // planes, cut
   if (rk_small_grid(c))
     for (int cut = kRkCutMax; cut > 1; cut /= 2) candidates.emplace_back(kRkChunks[0], cut);
-  for (int k : kRkChunks) candidates.emplace_back(k, 1);
+  for (int k : kRkChunks)
+    if (!rk_small_grid(c) || k <= 16) candidates.emplace_back(k, 1);
   int best_cut = 1;
   for (int v = 0; v < (tune_carry ? 2 : 1) && e == cudaSuccess; ++v) {
     if (tune_carry) c->rk2_carry = v == 1;

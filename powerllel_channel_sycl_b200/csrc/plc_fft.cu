@@ -263,6 +263,40 @@ struct Dft<3, INV> {
   }
 };
 
+// 9-point DFT as three 3-point DFTs of the interleaved subsequences x[3m + r],
+// the twiddles W9^(r k), and three 3-point DFTs across r:
+// X[k + 3q] = sum_r W3^(r q) W9^(r k) Y_r[k], W9 = exp(-+ 40 deg i)
+template <bool INV>
+struct Dft<9, INV> {
+  template <class V>
+  __device__ __forceinline__ static void run(V (&v)[9]) {
+    using S = ScalarOf<V>;
+    // cos and sin of 40, 80 and 160 degrees
+    const V w1 = mk<V>(S(0.76604444311897803520), S(-0.64278760968653932632));
+    const V w2 = mk<V>(S(0.17364817766693034885), S(-0.98480775301220805937));
+    const V w4 = mk<V>(S(-0.93969262078590838405), S(-0.34202014332566873304));
+    V y[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+#pragma unroll
+      for (int m = 0; m < 3; ++m) y[r][m] = v[3 * m + r];
+      Dft<3, INV>::run(y[r]);
+    }
+    y[1][1] = INV ? cmulc(y[1][1], w1) : cmul(y[1][1], w1);
+    y[1][2] = INV ? cmulc(y[1][2], w2) : cmul(y[1][2], w2);
+    y[2][1] = INV ? cmulc(y[2][1], w2) : cmul(y[2][1], w2);
+    y[2][2] = INV ? cmulc(y[2][2], w4) : cmul(y[2][2], w4);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      V t[3] = {y[0][k], y[1][k], y[2][k]};
+      Dft<3, INV>::run(t);
+      v[k] = t[0];
+      v[k + 3] = t[1];
+      v[k + 6] = t[2];
+    }
+  }
+};
+
 // 24-point DFT as three 8-point DFTs of the interleaved subsequences
 // x[3m + r], the twiddles W24^(r k), and eight 3-point DFTs across r:
 // X[k + 8q] = sum_r W3^(r q) W24^(r k) Y_r[k] (Cooley-Tukey with n = 3m + r,
@@ -347,12 +381,17 @@ __device__ __forceinline__ void fft_pass(const V *__restrict__ src, V *__restric
   const int nb = n / R;
   const int tot = nl * nb;
   const int tws = n / (Ns * R);
+  // b / nb and j / Ns by reciprocals: (b + 1/2) / nb is at least 1/(2 nb) away from
+  // an integer and its relative error at most 2^-22, so the quotients are exact
+  // for b < 2^20; an integer division costs as much as a radix-3 butterfly
+  const float inv_nb = 1.f / (float)nb, inv_Ns = 1.f / (float)Ns;
   for (int b = threadIdx.x; b < tot; b += blockDim.x) {
-    const int l = b / nb;
+    const int l = (int)(((float)b + 0.5f) * inv_nb);
     const int j = b - l * nb;
     const V *s = src + l * LS;
     V *d = dst + l * LS;
-    const int jm = j % Ns;
+    const int jq = (int)(((float)j + 0.5f) * inv_Ns);
+    const int jm = j - jq * Ns;
     V v[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) v[r] = s[padi<V>(j + r * nb)];
@@ -364,7 +403,7 @@ __device__ __forceinline__ void fft_pass(const V *__restrict__ src, V *__restric
       }
     }
     Dft<R, INV>::run(v);
-    const int idxD = (j / Ns) * Ns * R + jm;
+    const int idxD = jq * Ns * R + jm;
 #pragma unroll
     for (int r = 0; r < R; ++r) d[padi<V>(idxD + r * Ns)] = v[r];
   }
@@ -381,6 +420,7 @@ __device__ V *fft_run(V *A, V *B, int nl, int LS, const FftDev<V> &P) {
       case 8: fft_pass<8, INV>(A, B, nl, P.n, LS, Ns, P.tw); break;
       case 4: fft_pass<4, INV>(A, B, nl, P.n, LS, Ns, P.tw); break;
       case 2: fft_pass<2, INV>(A, B, nl, P.n, LS, Ns, P.tw); break;
+      case 9: fft_pass<9, INV>(A, B, nl, P.n, LS, Ns, P.tw); break;
       default: fft_pass<3, INV>(A, B, nl, P.n, LS, Ns, P.tw); break;
     }
     __syncthreads();
@@ -393,7 +433,8 @@ __device__ V *fft_run(V *A, V *B, int nl, int LS, const FftDev<V> &P) {
 }
 
 // ---------------------------------------------------------------------------
-// Compile-time plans.  For the line lengths of the supported grids the radix
+// Compile-time plans.  For the line lengths of the supported grids, all with at
+// most one factor 3, the radix
 // sequence (the rule of host_fft_factor: 16s, then one 8/4/2, then 3s) and
 // all index arithmetic are constants, the passes are unrolled and the
 // integer divisions become multiplications; N = 0 selects the runtime plan.
