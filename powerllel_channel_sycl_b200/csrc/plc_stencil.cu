@@ -1104,29 +1104,60 @@ __global__ void __launch_bounds__(BX *BY) k_force_apply(Geo g, const StepConst *
   }
 }
 
-// Boundary update of the velocity (mod_updateBound.cc:263-285) as one kernel
-// over the interior: every interior point rewrites its own halo images.
+// The interior points that own a halo image or a wall ghost, numbered: the two
+// wall planes, then the first and last rows of the others, then the first and
+// last points of the other rows.  The boundary updates launch one thread per such
+// point, not per interior point (of 192 x 96 x 96, 87 thousand of 1.8 million).
+struct BoundPoints {
+  int nx, ny, nz;
+  __host__ __device__ int walls() const { return 2 * nx * ny; }
+  __host__ __device__ int rows() const { return 2 * nx * (nz - 2); }
+  __host__ __device__ int ends() const { return 2 * (ny - 2) * (nz - 2); }
+  __host__ __device__ int count() const { return walls() + rows() + ends(); }
+  __device__ __forceinline__ void at(int e, int &i, int &j, int &k) const {
+    if (e < walls()) {
+      const int r = e / nx;
+      i = e - r * nx + 1;
+      j = r % ny + 1;
+      k = r < ny ? 1 : nz;
+    } else if (e < walls() + rows()) {
+      const int q = e - walls(), r = q / nx;
+      i = q - r * nx + 1;
+      j = r & 1 ? ny : 1;
+      k = (r >> 1) + 2;
+    } else {
+      const int q = e - walls() - rows(), r = q >> 1;
+      i = q & 1 ? nx : 1;
+      k = r / (ny - 2);
+      j = r - k * (ny - 2) + 2;
+      k += 2;
+    }
+  }
+};
+
+// Boundary update of the velocity (mod_updateBound.cc:263-285) as one kernel:
+// every point that owns an image rewrites its own halo images.
 template <class T>
 __global__ void __launch_bounds__(BX *BY) k_bound_vel(Geo g, double u_crf, T *u, T *v, T *w) {
-  const int i = blockIdx.x * BX + threadIdx.x + 1;
-  const int j = blockIdx.y * BY + threadIdx.y + 1;
-  const int k = blockIdx.z + 1;
-  if (i > g.nx || j > g.ny) return;
-  // only points that own an image do any work
-  if (!(i == 1 || i == g.nx || j == 1 || j == g.ny || k == 1 || k == g.nz)) return;
+  const BoundPoints b{g.nx, g.ny, g.nz};
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= b.count()) return;
+  int i, j, k;
+  b.at(e, i, j, k);
   const long long c = g.at(i, j, k);
-  store_with_halo(u, g, i, j, k, u[c], BC_CENTRED, T(0.0 - u_crf));
-  store_with_halo(v, g, i, j, k, v[c], BC_CENTRED, T(0));
-  store_with_halo(w, g, i, j, k, w[c], BC_FACE, T(0));
+  const T uc = u[c], vc = v[c], wc = w[c];
+  store_with_halo(u, g, i, j, k, uc, BC_CENTRED, T(0.0 - u_crf));
+  store_with_halo(v, g, i, j, k, vc, BC_CENTRED, T(0));
+  store_with_halo(w, g, i, j, k, wc, BC_FACE, T(0));
 }
 
 template <class T>
 __global__ void __launch_bounds__(BX *BY) k_bound_p(Geo g, T *p) {
-  const int i = blockIdx.x * BX + threadIdx.x + 1;
-  const int j = blockIdx.y * BY + threadIdx.y + 1;
-  const int k = blockIdx.z + 1;
-  if (i > g.nx || j > g.ny) return;
-  if (!(i == 1 || i == g.nx || j == 1 || j == g.ny || k == 1 || k == g.nz)) return;
+  const BoundPoints b{g.nx, g.ny, g.nz};
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= b.count()) return;
+  int i, j, k;
+  b.at(e, i, j, k);
   store_with_halo(p, g, i, j, k, p[g.at(i, j, k)], BC_ZEROGRAD, T(0));
 }
 
@@ -1502,6 +1533,10 @@ inline dim3 interior_grid(const plc_ctx *c) {
   return dim3((c->nx + BX - 1) / BX, (c->ny + BY - 1) / BY, c->nz);
 }
 
+inline unsigned bound_grid(const plc_ctx *c) {
+  return (unsigned)((BoundPoints{c->nx, c->ny, c->nz}.count() + BX * BY - 1) / (BX * BY));
+}
+
 inline int reduce_blocks(const plc_ctx *c) {
   long long n = (long long)c->nx * c->ny * c->nz;
   long long b = (n + 255) / 256;
@@ -1747,21 +1782,21 @@ cudaError_t launch_mean_force(const plc_ctx *c, const double *u, cudaStream_t s)
 
 cudaError_t launch_bound_vel(const plc_ctx *c, double u_crf, double *u, double *v, double *w,
                              cudaStream_t s) {
-  k_bound_vel<double><<<interior_grid(c), dim3(BX, BY), 0, s>>>(c->geo(), u_crf, u, v, w);
+  k_bound_vel<double><<<bound_grid(c), BX * BY, 0, s>>>(c->geo(), u_crf, u, v, w);
   return cudaGetLastError();
 }
 cudaError_t launch_bound_vel(const plc_ctx *c, double u_crf, float *u, float *v, float *w,
                              cudaStream_t s) {
-  k_bound_vel<float><<<interior_grid(c), dim3(BX, BY), 0, s>>>(c->geo(), u_crf, u, v, w);
+  k_bound_vel<float><<<bound_grid(c), BX * BY, 0, s>>>(c->geo(), u_crf, u, v, w);
   return cudaGetLastError();
 }
 
 cudaError_t launch_bound_p(const plc_ctx *c, double *p, cudaStream_t s) {
-  k_bound_p<double><<<interior_grid(c), dim3(BX, BY), 0, s>>>(c->geo(), p);
+  k_bound_p<double><<<bound_grid(c), BX * BY, 0, s>>>(c->geo(), p);
   return cudaGetLastError();
 }
 cudaError_t launch_bound_p(const plc_ctx *c, float *p, cudaStream_t s) {
-  k_bound_p<float><<<interior_grid(c), dim3(BX, BY), 0, s>>>(c->geo(), p);
+  k_bound_p<float><<<bound_grid(c), BX * BY, 0, s>>>(c->geo(), p);
   return cudaGetLastError();
 }
 
