@@ -221,6 +221,28 @@ cudaError_t extract_t(const plc_ctx *c, int field, int dir, int3 st, int3 sz, do
 
 using namespace plc;
 
+namespace {
+// Device memory for n values of a profile: the context's reduction scratch,
+// which only work on the context's stream uses, or, for more planes than it
+// holds, an allocation of its own.  (A stream-ordered allocation per call went
+// back to the system at the call's synchronisation: 0.1 to several ms a call.)
+struct ProfileBuffer {
+  plc_ctx *c;
+  double *d = nullptr;
+  bool own = false;
+  ProfileBuffer(plc_ctx *ctx, size_t n) : c(ctx) {
+    own = n > (size_t)8 * kMaxBlocksReduce;
+    if (!own)
+      d = c->d_partials;
+    else if (cudaMallocAsync(&d, n * sizeof(double), c->stream) != cudaSuccess)
+      d = nullptr;
+  }
+  ~ProfileBuffer() {
+    if (own && d) cudaFreeAsync(d, c->stream);
+  }
+};
+}  // namespace
+
 extern "C" {
 
 // ---- mod_statistics -------------------------------------------------------
@@ -310,36 +332,29 @@ int plc_stat_profiles(plc_ctx *c, double *h_prof) {
   PLC_NEED_STAT(c);
   if (!h_prof) return set_error(c, PLC_ERR_ARG, "null destination");
   const size_t n = (size_t)kStatVars * c->nz;
-  double *d = nullptr;
-  PLC_CUDA(c, cudaMallocAsync(&d, n * sizeof(double), c->stream));
+  const ProfileBuffer buf(c, n);
+  if (!buf.d) return set_error(c, PLC_ERR_NOMEM, "profile buffer");
   k_stat_profiles<<<dim3(c->nz, kStatVars), 256, 0, c->stream>>>(
-      c->nx, c->ny, c->nz, stat_sums(c), c->stat_nspl > 0 ? 1.0 / c->stat_nspl : 0.0, d);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(h_prof, d, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-  const cudaError_t ef = cudaFreeAsync(d, c->stream);
-  if (e == cudaSuccess) e = ef;
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return cuda_status(c, e, "plc_stat_profiles");
+      c->nx, c->ny, c->nz, stat_sums(c), c->stat_nspl > 0 ? 1.0 / c->stat_nspl : 0.0, buf.d);
+  PLC_LAUNCH(c, "plc_stat_profiles");
+  PLC_CUDA(c, cudaMemcpyAsync(h_prof, buf.d, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  PLC_CUDA(c, cudaStreamSynchronize(c->stream));
   return PLC_OK;
 }
 
 int plc_mean_profile(plc_ctx *c, double *h_prof) {
   PLC_CHECK_CTX(c);
   if (!h_prof) return set_error(c, PLC_ERR_ARG, "null destination");
-  double *d = nullptr;
-  PLC_CUDA(c, cudaMallocAsync(&d, c->nz * sizeof(double), c->stream));
+  const ProfileBuffer buf(c, (size_t)c->nz);
+  if (!buf.d) return set_error(c, PLC_ERR_NOMEM, "profile buffer");
+  double *d = buf.d;
   if (c->mixed)
     k_plane_mean<float><<<c->nz, 256, 0, c->stream>>>(c->geo(), c->f_field[PLC_U], c->prm.u_crf, d);
   else
     k_plane_mean<double><<<c->nz, 256, 0, c->stream>>>(c->geo(), c->d_field[PLC_U], c->prm.u_crf, d);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(h_prof, d, c->nz * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-  const cudaError_t ef = cudaFreeAsync(d, c->stream);
-  if (e == cudaSuccess) e = ef;
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-  if (e != cudaSuccess) return cuda_status(c, e, "plc_mean_profile");
+  PLC_LAUNCH(c, "plc_mean_profile");
+  PLC_CUDA(c, cudaMemcpyAsync(h_prof, d, c->nz * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  PLC_CUDA(c, cudaStreamSynchronize(c->stream));
   return PLC_OK;
 }
 
