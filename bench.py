@@ -64,7 +64,7 @@ WORKLOADS = {
 # counted once (halos and 1-D coefficients excluded).
 KERNEL_BYTES_PER_POINT = {
     "rk1+bound(u1)": 48,          # read u,v,w; write u1,v1,w1
-    "rk2+bound(u)+mean": 72,      # read u1,v1,w1,u,v,w; write u,v,w
+    "rk2+bound(u)+mean": 80,      # read u1,v1,w1,u,v,w; write u,v,w; read u (mean)
     "calcRHS+fft_x_fwd": 32,      # read u,v,w; write spectral array
     "fft_y_fwd": 16,              # spectral array in place
     "trid_z": 16,                 # spectral array in place (pivot table excluded)
@@ -72,7 +72,7 @@ KERNEL_BYTES_PER_POINT = {
     "fft_x_bwd+bound(p)": 16,     # read spectral array; write p
     "correct+force+bound(u)": 56,  # read p,u,v,w; write u,v,w
 }
-STEP_BYTES_PER_POINT = sum(KERNEL_BYTES_PER_POINT.values())  # 272
+STEP_BYTES_PER_POINT = sum(KERNEL_BYTES_PER_POINT.values())  # 280
 # the mixed form stores every field in FP32 (half the bytes; the pivot table
 # excluded, as above)
 MIXED_BYTES_PER_POINT = {

@@ -166,7 +166,8 @@ int plc_field_ptr_f32(plc_ctx *ctx, int field, float **d_ptr, size_t *count, int
 int plc_fft_tiles(const plc_ctx *ctx, int *lines_xf, int *lines_x, int *lines_y);
 /* The plan family of the (backward) x and the y transforms, timed per
  * context with the tiles where a length has more than one (0: radix 16, one
- * 8/4/2, then 3s; 1: for lengths 3 * 2^a with 3 <= a <= 7, two passes
+ * 8/4/2, then 3s, pairs of them as radix 9 where the plan is not compiled
+ * per length; 1: for lengths 3 * 2^a with 3 <= a <= 7, two passes
  * ending in a radix-24 butterfly; 2: warp-line kernels, groups of four
  * warps transforming their own lines with no block barrier, for lengths
  * 32, 48, 64, 96, 128, 192, 256, 384, 512, 768; 3, y lines only: two passes
@@ -183,7 +184,8 @@ int plc_fft_plan_x_fwd(const plc_ctx *ctx, int *plan);
 /* z planes per block of the two RK stages, timed per context at creation
  * among 8, 16, 24 and 32 (at most nz) on both fused stages (on a grid whose
  * 8-plane blocks do not fill the device, a block may take a half or a quarter
- * of them); PLC_RK_KCHUNK (FP64 form) and PLC_RK_KCHUNK_F32 (mixed form) pin it.  The choice changes speed; results only in the mixed form, whose
+ * of them); PLC_RK_KCHUNK (FP64 form) and PLC_RK_KCHUNK_F32 (mixed form)
+ * pin it.  The choice changes speed; results only in the mixed form, whose
  * RK2 sums the bulk mean per block in FP32 (by FP32 rounding).  No
  * counterpart in the reference. */
 int plc_rk_kchunk(const plc_ctx *ctx, int *kchunk);

@@ -16,9 +16,10 @@
 //    (calcRHS fused, mod_calcRHS.cc:23-30).
 //  * y lines pair adjacent packed-x columns i, i+1 and are read and written in
 //    place with x-contiguous row segments: no transpose buffer.
-//  * The complex FFT is a mixed-radix (16, 8, 4, 2, 3) Stockham transform between
-//    two shared-memory buffers, one butterfly per thread and pass; element e
-//    of a line lives at e + e/8 (FP64) or e + e/16 (FP32) to spread the
+//  * The complex FFT is a mixed-radix (16, 8, 4, 2, 3; 9 in plans not
+//    compiled per length) Stockham transform between two shared-memory
+//    buffers, one butterfly per thread and pass; element e of a line lives at
+//    e + e/8 (FP64) or e + e/16 (FP32) to spread the
 //    strided accesses over the banks.
 //  * Both transforms are unscaled; the backward x transform multiplies by
 //    1/(nx*ny) (mod_fft.cc:57,116-117) and, in the fused step, also writes

@@ -945,8 +945,10 @@ __global__ void __launch_bounds__(256, 2) k_correct_fused(Geo g, StepConst *sc, 
 }
 
 // The fused correction of the mixed form, and of the FP64 form where it is forced
-// in x alone (correction and forcing 0.90 + 0.21 -> 0.67 ms there): correctVel (mod_calcVel.cc:272-274) plus the forcing sc->force[d]
-// that has already been reduced (0 for unforced components), written with the halo images and wall ghosts.
+// in x alone (correction and forcing 0.90 + 0.21 -> 0.67 ms there): correctVel
+// (mod_calcVel.cc:272-274) plus the forcing sc->force[d] that has already been
+// reduced (0 for unforced components), written with the halo images and wall
+// ghosts.
 // No reduction, so a plain grid: each thread takes KZ planes of one column
 // (p(k+1) of a plane is p(k) of the next) with all loads issued first.  The halo
 // images are stored inline, predicated per lane (out of line, off the common path:
