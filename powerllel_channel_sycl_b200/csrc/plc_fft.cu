@@ -2402,7 +2402,6 @@ static_assert(sizeof(XfBatch) <= 32000 && sizeof(YBatch) <= 32000 && sizeof(XbBa
 // thomas_inplace.  Every wait is bounded: on a timeout the block records
 // the error word and leaves.
 // ---------------------------------------------------------------------------
-constexpr int kTridChunks = 8;
 constexpr long long kTridWaitLimit = 1ll << 22;
 
 __device__ __forceinline__ unsigned trid_smem_addr(const void *p) {
@@ -2427,8 +2426,6 @@ __device__ __forceinline__ bool trid_try_wait(unsigned long long *bar) {
       : "memory");
   return ok != 0;
 }
-
-size_t trid_tile_smem(int nz, size_t elem) { return (size_t)nz * 32 * elem + 8 * kTridChunks + 16; }
 
 // The block's columns: systems t = blockIdx.x * 32 + lane (nx % 32 == 0, so
 // one packed y row j); xs[k * 32 + lane] holds row k of the lane's system.
@@ -3285,17 +3282,11 @@ cudaError_t fft_set_lines(plc_ctx *c, int lines_xf, int lines_x, int lines_y) {
                   : fft_grids_t<double>(c, (size_t)dev_max, sms);
 }
 
-// The on-chip sweep needs whole 32-system rows (nx a multiple of 32) and its
-// columns within the device's shared memory; else the streaming sweep runs.
-static bool trid_tile_ok(const plc_ctx *c, size_t elem) {
-  return c->trid_tile && c->nx % 32 == 0 && trid_tile_smem(c->nz, elem) <= c->trid_smem_max;
-}
 cudaError_t launch_trid(const plc_ctx *c, double *var, cudaStream_t s) {
-  if (c->trid_split && trid_split_ok(c->nz) &&
-      reinterpret_cast<unsigned long long>(var) % (2 * sizeof(double)) == 0)
-    return launch_trid_split(c, var, s);
+  const TridSweep sweep = trid_sweep(c, sizeof(double), var);
+  if (sweep == TRID_SPLIT) return launch_trid_split(c, var, s);
   const long long plane = (long long)c->nx * c->ny;
-  if (trid_tile_ok(c, sizeof(double))) {
+  if (sweep == TRID_TILE) {
     k_trid_tile<<<(unsigned)(plane / 32), 32, trid_tile_smem(c->nz, sizeof(double)), s>>>(
         c->nx, c->ny, c->nz, c->d_rpiv, c->d_ac, c->d_ac + c->nz, var, c->d_err);
     return cudaGetLastError();
@@ -3306,11 +3297,10 @@ cudaError_t launch_trid(const plc_ctx *c, double *var, cudaStream_t s) {
   return cudaGetLastError();
 }
 cudaError_t launch_trid(const plc_ctx *c, float *var, cudaStream_t s) {
-  if (c->trid_split && trid_split_ok(c->nz) &&
-      reinterpret_cast<unsigned long long>(var) % (2 * sizeof(float)) == 0)
-    return launch_trid_split(c, var, s);
+  const TridSweep sweep = trid_sweep(c, sizeof(float), var);
+  if (sweep == TRID_SPLIT) return launch_trid_split(c, var, s);
   const long long plane = (long long)c->nx * c->ny;
-  if (trid_tile_ok(c, sizeof(float))) {
+  if (sweep == TRID_TILE) {
     k_trid_mixed_tile<<<(unsigned)(plane / 32), 32, trid_tile_smem(c->nz, sizeof(float)), s>>>(
         c->nx, c->ny, c->nz, c->d_rpiv32, c->d_ac32, c->d_ac32 + c->nz, c->d_rpiv, c->d_ac,
         c->d_ac + c->nz, var, c->d_low, c->d_err);

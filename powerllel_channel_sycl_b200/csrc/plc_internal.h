@@ -263,9 +263,8 @@ cudaError_t launch_fft_y(const plc_ctx *c, float *var, bool inverse,
 cudaError_t launch_trid(const plc_ctx *c, double *var, cudaStream_t s);
 cudaError_t launch_trid(const plc_ctx *c, float *var, cudaStream_t s);
 // the sweep with each column split over the threads of a block (plc_trid.cu),
-// for columns of trid_split_ok(nz) planes; spectral arrays not aligned to a
-// pair of elements take the streaming sweep
-bool trid_split_ok(int nz);
+// for columns of trid_split_ok(nz) planes; launch_trid takes it, or a serial
+// sweep, by trid_sweep()
 cudaError_t launch_trid_split(const plc_ctx *c, double *var, cudaStream_t s);
 cudaError_t launch_trid_split(const plc_ctx *c, float *var, cudaStream_t s);
 cudaError_t launch_check(const plc_ctx *c, const double *u, const double *v,
@@ -410,6 +409,29 @@ bool step_needs_host(const plc_ctx *c);
 // closes the monitor files and releases the I/O state (plc_io.cc)
 void io_free(plc_ctx *c);
 
+// Tallest column of the split sweep: 16 segments of 16 planes in registers
+constexpr int kTridSplitMax = 256;
+inline bool trid_split_ok(int nz) { return nz <= kTridSplitMax; }
+// Chunks of planes, each with a barrier, in which the on-chip sweep copies its
+// columns, and its shared memory (32 columns and the barriers)
+constexpr int kTridChunks = 8;
+inline size_t trid_tile_smem(int nz, size_t elem) {
+  return (size_t)nz * 32 * elem + 8 * kTridChunks + 16;
+}
+// The Thomas sweep of a solve of the spectral array `var` of elem-byte elements.
+// The split sweep loads pairs of elements and the on-chip sweep rows by bulk
+// copies from 16-byte boundaries; any other array takes the streaming sweep,
+// which loads single elements.  The on-chip sweep also needs whole rows of 32
+// systems and its columns within the device's shared memory.
+enum TridSweep { TRID_SPLIT, TRID_TILE, TRID_STREAM };
+inline TridSweep trid_sweep(const plc_ctx *c, size_t elem, const void *var) {
+  const size_t at = reinterpret_cast<size_t>(var);
+  if (c->trid_split && trid_split_ok(c->nz) && at % (2 * elem) == 0) return TRID_SPLIT;
+  if (c->trid_tile && c->nx % 32 == 0 && at % 16 == 0 &&
+      trid_tile_smem(c->nz, elem) <= c->trid_smem_max)
+    return TRID_TILE;
+  return TRID_STREAM;
+}
 inline int rk_chunk(const plc_ctx *c, int kmax) {
   int k = c->rk_kchunk > 0 ? c->rk_kchunk : kmax;
   if (k > kmax) k = kmax;

@@ -329,7 +329,7 @@ static_assert(sizeof(SplitBatch) <= 32000, "kernel parameters are limited to 327
 
 // compiled segment lengths
 __host__ __device__ __forceinline__ int split_ch(int np) { return np <= 4 ? 4 : (np <= 8 ? 8 : 16); }
-constexpr int kSplitMax = 16 * kSeg;  // tallest column
+static_assert(kTridSplitMax == 16 * kSeg, "the longest compiled segment is 16 planes");
 
 template <int CHMAX>
 __global__ void __launch_bounds__(kThreads, split_resident(CHMAX))
@@ -374,8 +374,6 @@ void split_dispatch(int nz, F &&f) {
 }
 
 }  // namespace
-
-bool trid_split_ok(int nz) { return nz <= kSplitMax; }
 
 cudaError_t launch_trid_split(const plc_ctx *c, double *var, cudaStream_t s) {
   split_dispatch(c->nz, [&](auto CH) {

@@ -77,6 +77,29 @@ def test_split_sweep_fp64(monkeypatch, nx, ny, nz):
     assert rel_l2(got["split"][:, 0, 0], got["stream"][:, 0, 0]) < 1e-9
 
 
+@pytest.mark.parametrize("mode", [None, "split", "tile", "stream"])
+@pytest.mark.parametrize("nx,ny,nz", [(32, 24, 2), (64, 48, 64), (36, 6, 10), (32, 6, 258)])
+def test_unaligned_array_is_streamed(monkeypatch, nx, ny, nz, mode):
+    """An array one element off a 16-byte boundary, whatever the context's sweep: the
+    streaming sweep's solution bit for bit."""
+    from powerllel_channel_sycl_b200 import Channel
+    var = np.random.default_rng(nx).standard_normal((nz, ny, nx))
+    ch = channel(monkeypatch, "stream", nx, ny, nz)
+    ch.upload("spec", var)
+    ch.solve_trid()
+    ref = ch.download("spec")
+    ch.close()
+    monkeypatch.setenv("PLC_TRID", mode) if mode else monkeypatch.delenv("PLC_TRID")
+    with Channel(channel_params(**case_kwargs(nx, ny, nz))) as ch:
+        field = np.zeros(ch.shape)
+        field.ravel()[1:1 + var.size] = var.ravel()
+        ch.upload("u1", field)
+        ch.solve_trid(ch.ptr("u1") + 8)
+        got = ch.download("u1").ravel()
+    np.testing.assert_array_equal(got[1:1 + var.size].reshape(var.shape), ref)
+    assert got[0] == 0.0 and not got[1 + var.size:].any()
+
+
 @pytest.mark.parametrize("nx,ny,nz", [s for s in SIZES if s[0] % 4 == 0 and s[1] % 4 == 0])
 def test_split_sweep_mixed(monkeypatch, nx, ny, nz):
     monkeypatch.setenv("PLC_FFT_PLANS_F32", "0,0")
