@@ -3608,6 +3608,71 @@ cudaError_t launch_fft_x_bwd_batch(plc_ctx *const *cs, int n, const BatchPlan *b
   return cudaSuccess;
 }
 
+namespace {
+// the channels whose own solves take the split sweep (split), or do not
+std::vector<plc_ctx *> trid_members(plc_ctx *const *cs, int n, bool split) {
+  std::vector<plc_ctx *> out;
+  for (int m = 0; m < n; ++m)
+    if ((trid_sweep(cs[m], sizeof(float), cs[m]->f_field[PLC_SPEC]) == TRID_SPLIT) == split)
+      out.push_back(cs[m]);
+  return out;
+}
+
+// whether every channel admits the on-chip sweep (whole blocks of 32 systems,
+// its column in shared memory)
+bool trid_tile_batch_ok(const std::vector<plc_ctx *> &cs) {
+  for (const plc_ctx *c : cs)
+    if (c->nx % 32 || trid_tile_smem(c->nz, sizeof(float)) > c->trid_smem_max) return false;
+  return !cs.empty();
+}
+
+cudaError_t launch_trid_tile_batch(const std::vector<plc_ctx *> &cs, cudaStream_t s, bool pdl) {
+  const int n = (int)cs.size();
+  for (int q0 = 0; q0 < n; q0 += kBatchMax) {
+    TrtBatch b;
+    std::memset(&b, 0, sizeof b);
+    b.n = std::min(kBatchMax, n - q0);
+    int tot = 0, nzmax = 0;
+    for (int q = 0; q < b.n; ++q) {
+      const plc_ctx *c = cs[q0 + q];
+      b.m[q] = TrtMember{c->nx,     c->ny,     c->nz,           c->d_rpiv32, c->d_ac32,
+                         c->d_ac32 + c->nz, c->d_rpiv, c->d_ac, c->d_ac + c->nz,
+                         c->f_field[PLC_SPEC], c->d_low, c->d_err};
+      b.start[q] = tot;
+      tot += (int)((long long)c->nx * c->ny / 32);
+      nzmax = std::max(nzmax, c->nz);
+    }
+    b.start[b.n] = tot;
+    const cudaError_t e = launch_batched(k_trid_mixed_tile_batch, (unsigned)tot, dim3(32),
+                                         trid_tile_smem(nzmax, sizeof(float)), s, b, pdl);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t launch_trid_stream_batch(const std::vector<plc_ctx *> &cs, cudaStream_t s, bool pdl) {
+  const int n = (int)cs.size();
+  for (int q0 = 0; q0 < n; q0 += kBatchMax) {
+    TrBatch b;
+    std::memset(&b, 0, sizeof b);
+    b.n = std::min(kBatchMax, n - q0);
+    int tot = 0;
+    for (int q = 0; q < b.n; ++q) {
+      const plc_ctx *c = cs[q0 + q];
+      b.m[q] = TrMember{c->nx,     c->ny,         c->nz,  c->d_rpiv32, c->d_ac32,
+                        c->d_ac32 + c->nz, c->d_rpiv, c->d_ac, c->d_ac + c->nz,
+                        c->f_field[PLC_SPEC], c->d_low};
+      b.start[q] = tot;
+      tot += (int)(((long long)c->nx * c->ny + 127) / 128);
+    }
+    b.start[b.n] = tot;
+    const cudaError_t e = launch_batched(k_trid_mixed_batch, (unsigned)tot, dim3(128), 0, s, b, pdl);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+}  // namespace
+
 // The batch autotuner: for every group of every batched transform, the
 // feasible families (only the channels' own where they are pinned) and
 // tiles, one untimed launch and the best of three timed ones each; then the
@@ -3666,19 +3731,22 @@ cudaError_t batch_autotune(plc_ctx *const *cs, int n, cudaStream_t s, BatchPlan 
       bp->dir[dir].push_back(best);
     }
   }
-  // the Thomas sweep where a channel does not have the split one: streamed, or
+  // the Thomas sweep of the channels that do not have the split one: streamed, or
   // with the columns on chip (as the channels have it where PLC_TRID pins it)
   bp->trid_tile = false;
+  const std::vector<plc_ctx *> serial = trid_members(cs, n, false);
   bool trid_pinned = false, trid_tiles = true;
-  for (int m = 0; m < n; ++m) {
-    trid_pinned = trid_pinned || cs[m]->trid_pinned;
-    trid_tiles = trid_tiles && cs[m]->trid_tile;
+  for (const plc_ctx *c : serial) {
+    trid_pinned = trid_pinned || c->trid_pinned;
+    trid_tiles = trid_tiles && c->trid_tile;
   }
   if (trid_pinned) {
-    bp->trid_tile = trid_tiles && trid_tile_batch_ok(cs, n);
-  } else if (!trid_split_batch_ok(cs, n) && trid_tile_batch_ok(cs, n)) {
-    const float ts = time_of([&]() { return launch_trid_batch(cs, n, false, s); });
-    const float tt = time_of([&]() { return launch_trid_batch(cs, n, true, s); });
+    bp->trid_tile = trid_tiles && trid_tile_batch_ok(serial);
+  } else if (trid_tile_batch_ok(serial)) {
+    plc_ctx *const *ser = serial.data();
+    const int ns = (int)serial.size();
+    const float ts = time_of([&]() { return launch_trid_batch(ser, ns, false, s); });
+    const float tt = time_of([&]() { return launch_trid_batch(ser, ns, true, s); });
     bp->trid_tile = tt >= 0.f && (ts < 0.f || tt < ts);
   }
   {
@@ -3704,57 +3772,15 @@ cudaError_t batch_autotune(plc_ctx *const *cs, int n, cudaStream_t s, BatchPlan 
   return cudaSuccess;
 }
 
-// whether every channel admits the on-chip sweep (whole blocks of 32 systems,
-// its column in shared memory)
-bool trid_tile_batch_ok(plc_ctx *const *cs, int n) {
-  for (int m = 0; m < n; ++m)
-    if (cs[m]->nx % 32 || trid_tile_smem(cs[m]->nz, sizeof(float)) > cs[m]->trid_smem_max)
-      return false;
-  return n > 0;
-}
-
 cudaError_t launch_trid_batch(plc_ctx *const *cs, int n, bool tile, cudaStream_t s, bool pdl) {
-  if (trid_split_batch_ok(cs, n)) return launch_trid_split_batch(cs, n, s, pdl);
-  if (tile && trid_tile_batch_ok(cs, n)) {
-    for (int q0 = 0; q0 < n; q0 += kBatchMax) {
-      TrtBatch b;
-      std::memset(&b, 0, sizeof b);
-      b.n = std::min(kBatchMax, n - q0);
-      int tot = 0, nzmax = 0;
-      for (int q = 0; q < b.n; ++q) {
-        const plc_ctx *c = cs[q0 + q];
-        b.m[q] = TrtMember{c->nx,     c->ny,     c->nz,           c->d_rpiv32, c->d_ac32,
-                           c->d_ac32 + c->nz, c->d_rpiv, c->d_ac, c->d_ac + c->nz,
-                           c->f_field[PLC_SPEC], c->d_low, c->d_err};
-        b.start[q] = tot;
-        tot += (int)((long long)c->nx * c->ny / 32);
-        nzmax = std::max(nzmax, c->nz);
-      }
-      b.start[b.n] = tot;
-      const cudaError_t e = launch_batched(k_trid_mixed_tile_batch, (unsigned)tot, dim3(32),
-                                           trid_tile_smem(nzmax, sizeof(float)), s, b, pdl);
-      if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
-  }
-  for (int q0 = 0; q0 < n; q0 += kBatchMax) {
-    TrBatch b;
-    std::memset(&b, 0, sizeof b);
-    b.n = std::min(kBatchMax, n - q0);
-    int tot = 0;
-    for (int q = 0; q < b.n; ++q) {
-      const plc_ctx *c = cs[q0 + q];
-      b.m[q] = TrMember{c->nx,     c->ny,         c->nz,  c->d_rpiv32, c->d_ac32,
-                        c->d_ac32 + c->nz, c->d_rpiv, c->d_ac, c->d_ac + c->nz,
-                        c->f_field[PLC_SPEC], c->d_low};
-      b.start[q] = tot;
-      tot += (int)(((long long)c->nx * c->ny + 127) / 128);
-    }
-    b.start[b.n] = tot;
-    const cudaError_t e = launch_batched(k_trid_mixed_batch, (unsigned)tot, dim3(128), 0, s, b, pdl);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  // each channel takes the sweep of its own solves, so that its results do not
+  // depend on the others': the split one in one launch, a serial one in another
+  const std::vector<plc_ctx *> split = trid_members(cs, n, true);
+  if (!split.empty())
+    if (cudaError_t e = launch_trid_split_batch(split.data(), (int)split.size(), s, pdl)) return e;
+  const std::vector<plc_ctx *> serial = trid_members(cs, n, false);
+  return tile && trid_tile_batch_ok(serial) ? launch_trid_tile_batch(serial, s, pdl)
+                                            : launch_trid_stream_batch(serial, s, pdl);
 }
 
 }  // namespace plc

@@ -322,7 +322,7 @@ struct BatchPlan {
   std::vector<Group> dir[3];  // BATCH_XF, BATCH_XB, BATCH_Y
   int rk_kchunk = 0;
   int rk_minb = 4;  // resident blocks per SM the RK kernels are compiled for (3 or 4)
-  bool trid_tile = false;  // the Thomas sweep with its columns on chip
+  bool trid_tile = false;  // the serial Thomas sweeps with their columns on chip
   // programmatic dependent launch: each batched kernel launched with
   // programmatic stream serialisation, so that its blocks become resident
   // while the kernels it depends on drain
@@ -354,13 +354,11 @@ cudaError_t launch_fft_x_fwd_batch(plc_ctx *const *cs, int n, const BatchPlan *b
                                    const cudaStream_t *ss, int ns);
 cudaError_t launch_fft_y_batch(plc_ctx *const *cs, int n, bool inverse, const BatchPlan *bp,
                                const cudaStream_t *ss, int ns);
+// each channel's own sweep (trid_sweep): the split sweeps in one launch, the serial
+// ones in another, on chip (tile) or streamed
 cudaError_t launch_trid_batch(plc_ctx *const *cs, int n, bool tile, cudaStream_t s,
                               bool pdl = false);
-// the batched split sweep, and whether every channel uses it
 cudaError_t launch_trid_split_batch(plc_ctx *const *cs, int n, cudaStream_t s, bool pdl);
-bool trid_split_batch_ok(plc_ctx *const *cs, int n);
-// whether every channel admits the batched on-chip Thomas sweep
-bool trid_tile_batch_ok(plc_ctx *const *cs, int n);
 cudaError_t launch_fft_x_bwd_batch(plc_ctx *const *cs, int n, const BatchPlan *bp,
                                    const cudaStream_t *ss, int ns);
 cudaError_t launch_correct_batch(plc_ctx *const *cs, int n, cudaStream_t s, bool pdl = false);

@@ -398,12 +398,6 @@ cudaError_t launch_trid_split(const plc_ctx *c, float *var, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-bool trid_split_batch_ok(plc_ctx *const *cs, int n) {
-  for (int m = 0; m < n; ++m)
-    if (!cs[m]->trid_split || !trid_split_ok(cs[m]->nz)) return false;
-  return n > 0;
-}
-
 cudaError_t launch_trid_split_batch(plc_ctx *const *cs, int n, cudaStream_t s, bool pdl) {
   for (int q0 = 0; q0 < n; q0 += kBatchMax) {
     SplitBatch b;

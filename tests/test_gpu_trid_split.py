@@ -118,14 +118,24 @@ def test_split_sweep_mixed(monkeypatch, nx, ny, nz):
     assert err["split"] <= 2 * err["stream"] + 2.0 ** -24, err
 
 
-def test_split_sweep_ensemble_matches_alone(monkeypatch):
-    """A member of a batched ensemble takes its own segment length, whatever
-    the other members' columns: the results are those of its own steps."""
+# members whose segments have each compiled length; a column above 256 planes on
+# chip or streamed as tuned, and one that only the streaming sweep takes, beside
+# short ones; a grid whose own solves take a lane per pair in both directions
+ENSEMBLES = [[(32, 24, 16), (36, 24, 54), (32, 32, 130), (24, 24, 250)],
+             [(32, 24, 16), (32, 32, 258), (36, 24, 54), (24, 24, 300)],
+             [(512, 288, 10), (32, 24, 16), (24, 24, 258)]]
+
+
+@pytest.mark.parametrize("chains", [1, 2])
+@pytest.mark.parametrize("sizes", ENSEMBLES)
+def test_split_sweep_ensemble_matches_alone(monkeypatch, sizes, chains):
+    """A member of a batched ensemble takes its own sweep and segment length,
+    whatever the other members' columns: the results are those of its own steps."""
     from powerllel_channel_sycl_b200 import Channel, Ensemble
     monkeypatch.setenv("PLC_FFT_PLANS_F32", "0,0")
     monkeypatch.setenv("PLC_RK_KCHUNK_F32", "8")
     prms = []
-    for nx, ny, nz in ((32, 24, 16), (36, 24, 54), (32, 32, 130), (24, 24, 250)):
+    for nx, ny, nz in sizes:
         p = channel_params(**case_kwargs(nx, ny, nz))
         p.precision = 1
         prms.append(p)
@@ -139,6 +149,7 @@ def test_split_sweep_ensemble_matches_alone(monkeypatch):
     ens = Ensemble(prms)
     ens.initFlow()
     ens.set_schedule("batched")
+    ens.set_batch_chains(chains)
     ens.step(3)
     for m, ref in zip(ens.members, alone):
         for f, r in zip("uvwp", ref):
