@@ -182,11 +182,12 @@ int plc_fft_plans(const plc_ctx *ctx, int *plan_x, int *plan_y);
  * timed separately from the backward one.  No counterpart in the reference. */
 int plc_fft_plan_x_fwd(const plc_ctx *ctx, int *plan);
 /* z planes per block of the two RK stages, timed per context at creation
- * among 8, 16, 24 and 32 (at most nz) on both fused stages (on a grid whose
- * 8-plane blocks do not fill the device, a block may take a half or a quarter
- * of them); PLC_RK_KCHUNK (FP64 form) and PLC_RK_KCHUNK_F32 (mixed form)
- * pin it.  The choice changes speed; results only in the mixed form, whose
- * RK2 sums the bulk mean per block in FP32 (by FP32 rounding).  No
+ * on both fused stages among 8, 16, 24 and 32, on a grid whose 8-plane blocks
+ * do not fill the device among 2, 4, 8 and 16 (at most nz).  PLC_RK_KCHUNK
+ * (FP64 form) and PLC_RK_KCHUNK_F32 (mixed form) pin it: any number from the
+ * smallest candidate of the grid to 32.  The choice changes speed; results
+ * only in the mixed form, whose RK2 sums the bulk mean per block in FP32 (by
+ * FP32 rounding): a run is repeated by pinning what this reports.  No
  * counterpart in the reference. */
 int plc_rk_kchunk(const plc_ctx *ctx, int *kchunk);
 /* Whether the mixed form's second RK stage carries its z-face terms from

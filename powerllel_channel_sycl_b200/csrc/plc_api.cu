@@ -12,7 +12,6 @@
 #include <new>
 #include <string>
 #include <type_traits>
-#include <utility>
 #include <vector>
 
 #include "plc_internal.h"
@@ -233,13 +232,13 @@ int run_check_fields(plc_ctx *c, int what) {
   return run_check(c, what, c->d_field[PLC_U], c->d_field[PLC_V], c->d_field[PLC_W]);
 }
 
-// Autotuner of the RK stages' z planes per block: each candidate of
-// kRkChunks (at most nz; on small grids also parts of the smallest) timed on both fused stages over the context's own
-// fields (best of three after a warm-up launch); the chunk changes which
-// blocks compute which planes: no result of the FP64 form, and in the mixed
-// form only the FP32 rounding of the per-block bulk-mean sums.  Run at
-// creation, before
-// the fields hold data to keep (the stages overwrite u1..w1 and u..w).
+// Autotuner of the RK stages' z planes per block: each candidate of kRkChunks
+// (small grids: kRkChunksSmall; at most nz) timed on both fused stages over the
+// context's own fields (best of three after a warm-up launch); the chunk
+// changes which blocks compute which planes: no result of the FP64 form, and in
+// the mixed form only the FP32 rounding of the per-block bulk-mean sums.  Run
+// at creation, before the fields hold data to keep (the stages overwrite
+// u1..w1 and u..w).
 cudaError_t rk_autotune(plc_ctx *c) {
   cudaEvent_t e0, e1;
   cudaError_t e = cudaEventCreate(&e0);
@@ -275,20 +274,12 @@ cudaError_t rk_autotune(plc_ctx *c) {
   // the mixed form's second stage with or without the z-face carry (unless
   // PLC_RK2_CARRY pins it), with every chunk
   const bool tune_carry = c->mixed && !c->rk2_carry_pinned;
-  // the cut chunks re-read a larger share of halo planes: only where the blocks
-  // do not fill the device
-  std::vector<std::pair<int, int>> candidates;  // planes, cut
-  if (rk_small_grid(c))
-    for (int cut = kRkCutMax; cut > 1; cut /= 2) candidates.emplace_back(kRkChunks[0], cut);
-  for (int k : kRkChunks)
-    if (!rk_small_grid(c) || k <= 16) candidates.emplace_back(k, 1);
-  int best_cut = 1;
+  const auto &candidates = rk_small_grid(c) ? kRkChunksSmall : kRkChunks;
   for (int v = 0; v < (tune_carry ? 2 : 1) && e == cudaSuccess; ++v) {
     if (tune_carry) c->rk2_carry = v == 1;
     int last = -1;
-    for (auto [k, cut] : candidates) {
+    for (int k : candidates) {
       c->rk_kchunk = k;
-      c->rk_cut = cut;
       const int eff = rk_chunk(c, 32);
       if (eff == last) continue;  // the same chunk once clamped to nz
       last = eff;
@@ -307,13 +298,11 @@ cudaError_t rk_autotune(plc_ctx *c) {
       if (best_t < 0.f || best < best_t) {
         best_t = best;
         best_k = k;
-        best_cut = cut;
         best_carry = c->rk2_carry;
       }
     }
   }
   c->rk_kchunk = best_k;
-  c->rk_cut = best_cut;
   c->rk2_carry = best_carry;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -725,9 +714,10 @@ int plc_create(const plc_params *prm, const double *h_dzf_global, int device, pl
   // PLC_RK_KCHUNK pins the RK stages' z planes per block instead of timing
   // the candidates
   if (const char *env = getenv(c->mixed ? "PLC_RK_KCHUNK_F32" : "PLC_RK_KCHUNK")) {
-    // at least the smallest candidate of all grids
+    // at least the smallest candidate of the grid: every chunk that the
+    // autotuner may choose can be pinned
     const int k = atoi(env);
-    if (k < kRkChunks[0] || k > 32)
+    if (k < rk_least_chunk(c) || k > 32)
       return fail(set_error(c, PLC_ERR_ARG, std::string("invalid PLC_RK_KCHUNK: ") + env));
     c->rk_kchunk = k;
     c->rk_pinned = true;
@@ -825,7 +815,7 @@ int plc_fft_plans(const plc_ctx *c, int *plan_x, int *plan_y) {
 
 int plc_rk_kchunk(const plc_ctx *c, int *kchunk) {
   if (!c || !kchunk) return set_error(nullptr, PLC_ERR_ARG, "null argument");
-  *kchunk = rk_chunk(c, 32) * c->rk_cut;
+  *kchunk = rk_chunk(c, 32);
   return PLC_OK;
 }
 

@@ -116,9 +116,9 @@ struct plc_ctx {
   bool trid_tile = true;
   bool trid_pinned = false;  // PLC_TRID = "split", "tile" or "stream"
   // z planes per block of the RK stages (0: the kernels' maximum), chosen by
-  // the autotuner among kRkChunks; PLC_RK_KCHUNK pins it
+  // the autotuner among kRkChunks, on small grids kRkChunksSmall;
+  // PLC_RK_KCHUNK pins it
   int rk_kchunk = 0;
-  int rk_cut = 1;          // 2 or 4: the blocks of a small grid take that part of it
   bool rk_pinned = false;  // PLC_RK_KCHUNK(_F32) set
   // mixed form: the second RK stage carries its z-face terms (at 3 blocks
   // per SM), chosen by the autotuner; PLC_RK2_CARRY pins it
@@ -195,11 +195,12 @@ int host_parse_param_json(const char *path, plc_params *prm, std::string &err);
 // RK z-chunk candidates and the chunk a launch uses (at most kmax and nz)
 constexpr int kRkChunks[4] = {8, 16, 24, 32};
 // On grids whose 8-plane blocks would not fill the device (32 x 24 x 16 has 4 of
-// them) the autotuner also cuts the 8 planes in 2 or 4: a block marches its
-// planes one after another, so there the chunk, not the arithmetic, sets the
-// stage's time.  FP64 128 x 64 x 64: 22 -> 19 us a stage (with event overhead),
-// mixed 18.6 -> 15.5; 32 x 24 x 16 in FP64 21 -> 12.
-constexpr int kRkCutMax = 4;
+// them; rk_small_grid) the autotuner tries 2 and 4 planes, and not 24 and 32: a
+// block marches its planes one after another, so there the chunk, not the
+// arithmetic, sets the stage's time.  FP64 128 x 64 x 64: 22 -> 19 us a stage (with
+// event overhead), mixed 18.6 -> 15.5; 32 x 24 x 16 in FP64 21 -> 12.  On the others
+// shorter chunks would only re-read a larger share of halo planes.
+constexpr int kRkChunksSmall[4] = {2, 4, 8, 16};
 inline int rk_chunk(const plc_ctx *c, int kmax);
 cudaError_t launch_rk(const plc_ctx *c, int stage, bool fuse_bc, double u_crf,
                       const double *qu, const double *qv, const double *qw,
@@ -433,7 +434,6 @@ inline TridSweep trid_sweep(const plc_ctx *c, size_t elem, const void *var) {
 inline int rk_chunk(const plc_ctx *c, int kmax) {
   int k = c->rk_kchunk > 0 ? c->rk_kchunk : kmax;
   if (k > kmax) k = kmax;
-  k /= c->rk_cut;
   return k < c->nz ? k : c->nz;
 }
 // FP64 form: the bulk mean is taken before the correction, which applies the force
@@ -447,6 +447,11 @@ inline bool forced_early(const plc_ctx *c) {
 inline bool rk_small_grid(const plc_ctx *c) {
   return (long long)((c->nx + 31) / 32) * ((c->ny + 15) / 16) * ((c->nz + 7) / 8) <
          2ll * (c->mixed ? 4 : 2) * c->device_sms;
+}
+// the least chunk that a pin may ask for: the least that the autotuner may choose
+inline int rk_least_chunk(const plc_ctx *c) {
+  const int k = rk_small_grid(c) ? kRkChunksSmall[0] : kRkChunks[0];
+  return k < c->nz ? k : c->nz;
 }
 
 }  // namespace plc

@@ -918,10 +918,10 @@ unsigned convert_blocks(const plc_ctx *c, long long n) {
 
 }  // namespace
 
-// Blocks of the FP32 RK grid at the smallest z chunk the autotuner may
-// choose (the capacity of the bulk-mean partials).
+// Blocks of the FP32 RK grid at the smallest z chunk of any grid (the capacity
+// of the bulk-mean partials).
 long long rk32_blocks(const plc_ctx *c) {
-  const int k0 = kRkChunks[0] / kRkCutMax, kchunk = c->nz < k0 ? c->nz : k0;
+  const int k0 = kRkChunksSmall[0], kchunk = c->nz < k0 ? c->nz : k0;
   return (long long)((c->nx + RX - 1) / RX) * ((c->ny + RY - 1) / RY) *
          ((c->nz + kchunk - 1) / kchunk);
 }

@@ -1,5 +1,6 @@
-"""The RK stages' z planes per block (autotuned among 8, 16, 24, 32; pinned
-by PLC_RK_KCHUNK / PLC_RK_KCHUNK_F32) change which blocks compute which planes: three fused
+"""The RK stages' z planes per block (autotuned among 8, 16, 24, 32, on grids
+whose 8-plane blocks do not fill the device among 2, 4, 8, 16; pinned by
+PLC_RK_KCHUNK / PLC_RK_KCHUNK_F32) change which blocks compute which planes: three fused
 steps of the FP64 form are bit-identical under every chunk, including one
 that does not divide nz.  The mixed form's fused RK2 also sums the bulk
 mean per block in FP32, so the chunk moves the forcing by FP32 rounding:
@@ -36,8 +37,8 @@ def run(monkeypatch, kchunk, precision, nx=64, ny=48, nz=40):
 @pytest.mark.parametrize("precision", [0, 1])
 def test_rk_chunk_changes_no_result(monkeypatch, precision):
     k_auto, ref = run(monkeypatch, None, precision)
-    assert k_auto in (8, 16, 24, 32)
-    for k in (8, 12, 32):
+    assert k_auto in (2, 4, 8, 16)
+    for k in (2, 4, 8, 12, 32):
         got_k, out = run(monkeypatch, k, precision)
         assert got_k == k
         for q, a, b in zip("uvwp", out, ref):
@@ -49,13 +50,29 @@ def test_rk_chunk_changes_no_result(monkeypatch, precision):
                 assert rel_l2(demean(a), demean(b)) <= 5e-3, (k, q)
 
 
-@pytest.mark.parametrize("value", ["0", "4", "33"])
-def test_rk_chunk_pin_rejected(monkeypatch, value):
-    """Pins outside 8..32 are refused (below 8 the mixed form's bulk-mean
-    partials would not hold the blocks)."""
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("size", [(32, 24, 2), (32, 24, 6), (32, 24, 16), (64, 48, 40),
+                                  (128, 64, 64), (256, 256, 80)])
+def test_reported_chunk_repeats_the_run(monkeypatch, size, precision):
+    """What the query reports is what the blocks march: pinned, it gives the
+    same run bit for bit, the mixed form's bulk mean included."""
+    monkeypatch.setenv("PLC_RK2_CARRY", "0")
+    k, ref = run(monkeypatch, None, precision, *size)
+    small = size != (256, 256, 80)
+    assert k in [min(c, size[2]) for c in ((2, 4, 8, 16) if small else (8, 16, 24, 32))]
+    got_k, out = run(monkeypatch, k, precision, *size)
+    assert got_k == k
+    for a, b in zip(out, ref):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("size,value", [((32, 24, 16), v) for v in ("-2", "0", "1", "33")] +
+                         [((256, 256, 80), v) for v in ("2", "7", "33")])
+def test_rk_chunk_pin_rejected(monkeypatch, size, value):
+    """Pins outside the grid's smallest candidate..32 are refused."""
     from powerllel_channel_sycl_b200 import Channel, PlcError
     monkeypatch.setenv("PLC_RK_KCHUNK_F32", value)
-    prm = channel_params(**case_kwargs(32, 24, 16))
+    prm = channel_params(**case_kwargs(*size))
     prm.precision = 1
     with pytest.raises(PlcError):
         Channel(prm)
