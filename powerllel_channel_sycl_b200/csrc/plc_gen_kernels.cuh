@@ -106,6 +106,35 @@ __device__ __forceinline__ bool tc_wait(unsigned long long *bar, unsigned parity
   return false;
 }
 
+// Tensor memory: the instructions are .sync.aligned, so that the lanes of a warp,
+// which may have parted at a predicate before, meet first.
+// cols columns, their address to *base (by one warp, which also gives them back)
+__device__ __forceinline__ void tc_alloc(unsigned *base, unsigned cols) {
+  __syncwarp();
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                   tc_smem_u32(base)),
+               "r"(cols));
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+}
+__device__ __forceinline__ void tc_dealloc(unsigned base, unsigned cols) {
+  __syncwarp();
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols));
+}
+// 16 columns from addr of the warp's 32 lanes (with the wait in one statement: no use
+// of the registers can be moved between the two)
+__device__ __forceinline__ void tc_ld16(unsigned addr, unsigned (&r)[16]) {
+  __syncwarp();
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+      "%14,%15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(addr)
+      : "memory");
+}
+
 // 16-byte asynchronous copy global -> shared; src_bytes 0 fills zeros
 __device__ __forceinline__ void tc_cp16(void *dst, const void *src, unsigned src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tc_smem_u32(dst)), "l"(src),
@@ -139,10 +168,7 @@ __global__ void __launch_bounds__(128) k_conv3d_tc(Shape s, const bf16 *__restri
       (reinterpret_cast<unsigned long long>(tc_smem) + 1023ull) & ~1023ull);
 
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     tc_smem_u32(&tmem_base_s)),
-                 "r"(kNCols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    tc_alloc(&tmem_base_s, kNCols);
   }
   if (t == 0) {
     for (int q = 0; q < kTcNB; ++q)
@@ -248,14 +274,7 @@ __global__ void __launch_bounds__(128) k_conv3d_tc(Shape s, const bf16 *__restri
     for (int c0 = 0; c0 < N; c0 += 16) {
       unsigned r[16];
       const unsigned addr = tmem + ((unsigned)(warp * 32) << 16) + (unsigned)c0;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-          "%14,%15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-            "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-            "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(addr));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      tc_ld16(addr, r);
       if (row < M) {
         float4 *dst = reinterpret_cast<float4 *>(Y + row * N + c0);
 #pragma unroll
@@ -273,7 +292,7 @@ __global__ void __launch_bounds__(128) k_conv3d_tc(Shape s, const bf16 *__restri
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kNCols));
+    tc_dealloc(tmem, kNCols);
   }
 }
 
@@ -326,10 +345,7 @@ __global__ void __launch_bounds__(128) k_conv3d_wgrad_tc(Shape s, const bf16 *__
       (reinterpret_cast<unsigned long long>(tc_smem) + 1023ull) & ~1023ull);
 
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     tc_smem_u32(&tmem_base_s)),
-                 "r"(kNCols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    tc_alloc(&tmem_base_s, kNCols);
   }
   if (t == 0) {
     for (int q = 0; q < kWgNB; ++q)
@@ -439,14 +455,7 @@ __global__ void __launch_bounds__(128) k_conv3d_wgrad_tc(Shape s, const bf16 *__
     for (int c0 = 0; c0 < N; c0 += 16) {
       unsigned r[16];
       const unsigned addr = tmem + ((unsigned)(warp * 32) << 16) + (unsigned)c0;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-          "%14,%15}, [%16];"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-            "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-            "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(addr));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      tc_ld16(addr, r);
       if (co < Co) {
         float *dst = dW + ((long long)tap * Co + co) * N + c0;
 #pragma unroll
@@ -461,7 +470,7 @@ __global__ void __launch_bounds__(128) k_conv3d_wgrad_tc(Shape s, const bf16 *__
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kNCols));
+    tc_dealloc(tmem, kNCols);
   }
 }
 
@@ -527,16 +536,6 @@ __device__ __forceinline__ void tc_commit(unsigned long long *bar) {
                    tc_smem_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ void tc_ld16(unsigned addr, unsigned (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
-      "%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(addr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 constexpr int tc_cols(int n) { return n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : (n <= 256 ? 256 : 512))); }
 
 constexpr int kHaloThreads = 256;
@@ -601,10 +600,7 @@ __global__ void __launch_bounds__(kHaloThreads) k_conv3d_halo(Shape s, const bf1
   }
 
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     tc_smem_u32(&tmem_base_s)),
-                 "r"(kCols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    tc_alloc(&tmem_base_s, kCols);
   }
   if (t == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem_u32(&bar)));
@@ -690,31 +686,33 @@ __global__ void __launch_bounds__(kHaloThreads) k_conv3d_halo(Shape s, const bf1
       for (int c0 = 0; c0 < NB; c0 += 16) {
         unsigned r[16];
         tc_ld16(tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)(mt * NB + c0), r);
-        if (!valid) continue;
-        if (o.pre) {
+        if (valid) {
+          if (o.pre) {
 #pragma unroll
-          for (int q = 0; q < 4; ++q)
-            reinterpret_cast<float4 *>(o.pre + at + c0)[q] =
-                make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
-                            __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
-        }
-        if (!o.film) continue;
-        float h[16];
+            for (int q = 0; q < 4; ++q)
+              reinterpret_cast<float4 *>(o.pre + at + c0)[q] =
+                  make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
+                              __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+          }
+          if (o.film) {
+            float h[16];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) h[q] = gam[c0 + q] * __uint_as_float(r[q]) + bet[c0 + q];
-        if (o.act) {
-          __align__(16) __nv_bfloat162 a[8];
+            for (int q = 0; q < 16; ++q) h[q] = gam[c0 + q] * __uint_as_float(r[q]) + bet[c0 + q];
+            if (o.act) {
+              __align__(16) __nv_bfloat162 a[8];
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
-            a[q] = __floats2bfloat162_rn(lrelu(h[2 * q]), lrelu(h[2 * q + 1]));
-          uint4 *dst = reinterpret_cast<uint4 *>(o.act + at + c0);
-          dst[0] = reinterpret_cast<const uint4 *>(a)[0];
-          dst[1] = reinterpret_cast<const uint4 *>(a)[1];
-        } else {
+              for (int q = 0; q < 8; ++q)
+                a[q] = __floats2bfloat162_rn(lrelu(h[2 * q]), lrelu(h[2 * q + 1]));
+              uint4 *dst = reinterpret_cast<uint4 *>(o.act + at + c0);
+              dst[0] = reinterpret_cast<const uint4 *>(a)[0];
+              dst[1] = reinterpret_cast<const uint4 *>(a)[1];
+            } else {
 #pragma unroll
-          for (int q = 0; q < 4; ++q)
-            reinterpret_cast<float4 *>(o.out + at + c0)[q] =
-                make_float4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+              for (int q = 0; q < 4; ++q)
+                reinterpret_cast<float4 *>(o.out + at + c0)[q] =
+                    make_float4(h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+            }
+          }
         }
       }
     }
@@ -728,7 +726,7 @@ __global__ void __launch_bounds__(kHaloThreads) k_conv3d_halo(Shape s, const bf1
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
+    tc_dealloc(tmem, kCols);
   }
 }
 
@@ -774,10 +772,7 @@ __global__ void __launch_bounds__(kHaloThreads + 32)
   const int buf_bytes = 256 * R + kWgM * CO * 2;
 
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     tc_smem_u32(&tmem_base_s)),
-                 "r"(kCols));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    tc_alloc(&tmem_base_s, kCols);
   }
   if (t == 0) {
     for (int q = 0; q < NB; ++q) {
@@ -912,7 +907,7 @@ __global__ void __launch_bounds__(kHaloThreads + 32)
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
+    tc_dealloc(tmem, kCols);
   }
 }
 
