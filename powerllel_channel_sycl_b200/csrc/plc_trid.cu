@@ -80,6 +80,14 @@ struct Share {
   A v[2][kSeg][2 * NS + 1][kLanes];
 };
 
+// Barrier of the block, reached by each warp at one of two places of the program
+// (solve_columns).  __syncthreads is defined where the whole block takes the
+// same path; the barrier by its number counts warps wherever they arrive.
+__device__ __forceinline__ void segment_barrier() {
+  __syncwarp();
+  asm volatile("barrier.cta.sync.aligned 0;" ::: "memory");
+}
+
 // The solve of one segment: n planes from k0 (FULL: n == CH; n <= 0: an
 // empty segment, E = 0 and M = 1).
 template <class T, class A, int NS, int CH, bool FULL>
@@ -127,7 +135,7 @@ __device__ __forceinline__ void solve_segment(const Lane<T, A> &L, long long pla
     for (int c = 0; c < C; ++c) sh.v[0][seg][c][lane] = e[c];
     sh.v[0][seg][C][lane] = m;
   }
-  __syncthreads();
+  segment_barrier();
   {
     A e[C];
 #pragma unroll
@@ -166,7 +174,7 @@ __device__ __forceinline__ void solve_segment(const Lane<T, A> &L, long long pla
     for (int c = 0; c < C; ++c) sh.v[1][seg][c][lane] = e[c];
     sh.v[1][seg][C][lane] = m;
   }
-  __syncthreads();
+  segment_barrier();
   {
     A e[C];
 #pragma unroll
@@ -214,7 +222,7 @@ __device__ __forceinline__ void solve_columns(const Lane<T, A> &L, int nz, long 
   const int np = split_planes(nz);
   const int k0 = (int)threadIdx.x / kLanes * np, n = min(np, nz - k0);
   Share<A, NS> &sh = *static_cast<Share<A, NS> *>(smem);
-  // (the two segments of a warp take the same side: both hold barriers)
+  // (the two segments of a warp take the same side: both hold the block's barriers)
   if (__all_sync(0xffffffffu, n == CH))
     solve_segment<T, A, NS, CH, true>(L, plane, row, PS, ca, cc, k0, n, sh);
   else
