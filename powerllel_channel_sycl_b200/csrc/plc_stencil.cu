@@ -836,7 +836,8 @@ __global__ void __launch_bounds__(BX *BY) k_correct(Geo g, const StepConst *__re
   w[c] -= (p[c + g.XY] - pc) * T(sc->dt) * T(__ldg(g.dzc_inv + k));
 }
 
-// Fused correction of the step: correctVel, the halo images of every
+// Fused correction of the FP64 step of a channel that is not forced in x alone
+// (forced_early): correctVel, the halo images of every
 // component that is not forced, and the bulk mean of every forced component
 // (after correction).  The last block turns the means into the forcing values
 // sc->force[d] = vel_force[d] - mean[d] (mod_calcVel.cc:280-301).
@@ -852,29 +853,21 @@ struct ForceCfg {
 // p(k+1) is read once for planes k and k+1 and ~6 loads per thread and plane
 // are in flight.  The block reduces once at the end (a reduction tail per
 // short-lived block would cost more than the correction itself).
-// T = double: the reference's arithmetic.  T = float (mixed form): the
-// correction in FP32, the bulk sums of the forced components in FP64.
-template <class T, int KZ>
+// The sums are double-double (the order-independent sum of the reference
+// restatement).
+template <int KZ>
 __global__ void __launch_bounds__(256, 2) k_correct_fused(Geo g, StepConst *sc, ForceCfg fc,
-                                                          const T *__restrict__ p, T *u, T *v,
-                                                          T *w, double *partials,
+                                                          const double *__restrict__ p, double *u,
+                                                          double *v, double *w, double *partials,
                                                           unsigned int *counter) {
   __shared__ double smem[2 * 3 * 32];
-  const T dtdxi = T(sc->dtdxi), dtdyi = T(sc->dtdyi), dt = T(sc->dt);
+  const double dtdxi = sc->dtdxi, dtdyi = sc->dtdyi, dt = sc->dt;
   const int tiles_x = (g.nx + 31) / 32, tiles_y = (g.ny + 7) / 8;
   const int per_chunk = tiles_x * tiles_y;
   const int items = per_chunk * ((g.nz + KZ - 1) / KZ);
   const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
   const long long X = g.X, XY = g.XY;
   DD s[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-  // FP64: error-free double-double terms (the order-independent sum of the
-  // reference restatement); FP32 fields: a plain FP64 sum of the FP32 values
-  auto acc = [](DD &a, double x) {
-    if constexpr (sizeof(T) == 8)
-      dd_add(a, x);
-    else
-      a.hi += x;
-  };
   for (int item = blockIdx.x; item < items; item += gridDim.x) {
     const int kc = item / per_chunk, r = item - kc * per_chunk;
     const int jt = r / tiles_x, it = r - jt * tiles_x;
@@ -883,7 +876,7 @@ __global__ void __launch_bounds__(256, 2) k_correct_fused(Geo g, StepConst *sc, 
     const int nk = min(KZ, g.nz - k0 + 1);
     const long long c0 = g.at(i, j, k0);
     const HaloCol h = halo_col(g, i, j);
-    T pc[KZ + 1], px[KZ], py[KZ], uu[KZ], vv[KZ], ww[KZ];
+    double pc[KZ + 1], px[KZ], py[KZ], uu[KZ], vv[KZ], ww[KZ];
 #pragma unroll
     for (int q = 0; q < KZ; ++q)
       if (q < nk) {
@@ -905,27 +898,27 @@ __global__ void __launch_bounds__(256, 2) k_correct_fused(Geo g, StepConst *sc, 
         const int k = k0 + q;
         const long long c = c0 + q * XY;
         // correctVel, mod_calcVel.cc:272-274
-        const T nu = uu[q] - (px[q] - pc[q]) * dtdxi;
-        const T nv = vv[q] - (py[q] - pc[q]) * dtdyi;
-        const T nw = ww[q] - (pc[q + 1] - pc[q]) * dt * T(__ldg(g.dzc_inv + k));
+        const double nu = uu[q] - (px[q] - pc[q]) * dtdxi;
+        const double nv = vv[q] - (py[q] - pc[q]) * dtdyi;
+        const double nw = ww[q] - (pc[q + 1] - pc[q]) * dt * __ldg(g.dzc_inv + k);
         const double dzl = __ldg(g.dzflzi + k);
         if (fc.forced[0]) {
           u[c] = nu;
-          acc(s[0], double(nu) * dzl);
+          dd_add(s[0], nu * dzl);
         } else {
-          store_point(u, g, h, c, k, nu, BC_CENTRED, T(0.0 - fc.u_crf));
+          store_point(u, g, h, c, k, nu, BC_CENTRED, 0.0 - fc.u_crf);
         }
         if (fc.forced[1]) {
           v[c] = nv;
-          acc(s[1], double(nv) * dzl);
+          dd_add(s[1], nv * dzl);
         } else {
-          store_point(v, g, h, c, k, nv, BC_CENTRED, T(0));
+          store_point(v, g, h, c, k, nv, BC_CENTRED, 0.0);
         }
         if (fc.forced[2]) {
           w[c] = nw;
-          acc(s[2], double(nw) * dzl);
+          dd_add(s[2], nw * dzl);
         } else {
-          store_point(w, g, h, c, k, nw, BC_FACE, T(0));
+          store_point(w, g, h, c, k, nw, BC_FACE, 0.0);
         }
       }
   }
@@ -1711,7 +1704,7 @@ cudaError_t correct_fused_t(const plc_ctx *c, const T *p, T *u, T *v, T *w, cuda
     long long nb = (long long)kBlocksPerSm * c->num_sms;
     if (nb > items) nb = items;
     if (nb > kMaxBlocksReduce) nb = kMaxBlocksReduce;
-    k_correct_fused<T, KZ><<<(unsigned)nb, 256, 0, s>>>(c->geo(), c->d_sc, force_cfg(c), p, u, v,
+    k_correct_fused<KZ><<<(unsigned)nb, 256, 0, s>>>(c->geo(), c->d_sc, force_cfg(c), p, u, v,
                                                        w, c->d_partials, c->d_counter);
   }
   return cudaGetLastError();
