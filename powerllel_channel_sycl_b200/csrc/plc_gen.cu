@@ -477,6 +477,7 @@ struct GenLayer {
 struct plc_gen {
   plc_gen_config cfg{};
   int device = 0;
+  int sms = 0;  // of the device
   cudaStream_t stream = nullptr;
   Shape lv[kLevels];
   std::vector<GenLayer> layers;
@@ -545,13 +546,13 @@ constexpr size_t kSmemMax = 225 * 1024;
 // parts of it that are multiples of 16) of which two blocks fit an SM and whose
 // blocks fill the device -- fewer channels read the input tile again --, else
 // the fewest if one block fits, else 0.
-int halo_channels(Shape s, int ci, int n) {
+int halo_channels(int sms, Shape s, int ci, int n) {
   const long long tiles = (long long)((s.Y * (s.X + 2) + kHaloM - 1) / kHaloM) * s.B * s.Z;
   int least = 0;
   for (int parts = 1; parts <= n / 16; ++parts) {
     if (n % parts || n / parts % 16) continue;
     const int nb = n / parts;
-    if (halo_smem(s.X, ci, nb) <= kSmemMax / 2 && tiles * parts >= 148) return nb;
+    if (halo_smem(s.X, ci, nb) <= kSmemMax / 2 && tiles * parts >= sms) return nb;
     if (halo_smem(s.X, ci, nb) <= kSmemMax) least = nb;
   }
   return least;
@@ -581,7 +582,7 @@ cudaError_t conv_tc(plc_gen *gn, Shape s, const bf16 *x, const bf16 *w, float *y
 int conv(plc_gen *gn, Shape s, const bf16 *x, const bf16 *w, const ConvOut &o, int ci, int co) {
   cudaError_t e;
   bool done = true;
-  switch (halo_channels(s, ci, co)) {
+  switch (halo_channels(gn->sms, s, ci, co)) {
     case 16: e = conv_halo<16>(gn, s, x, w, o, ci, co); break;
     case 32: e = conv_halo<32>(gn, s, x, w, o, ci, co); break;
     case 48: e = conv_halo<48>(gn, s, x, w, o, ci, co); break;
@@ -911,6 +912,7 @@ int plc_gen_create(const plc_gen_config *cfg, int device, plc_gen **out) {
   };
   cudaError_t e;
   if ((e = cudaSetDevice(device)) != cudaSuccess ||
+      (e = cudaDeviceGetAttribute(&gn->sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&gn->stream, cudaStreamNonBlocking)) != cudaSuccess) {
     gn->err = std::string("CUDA: ") + cudaGetErrorString(e);
     return fail(PLC_ERR_CUDA);
