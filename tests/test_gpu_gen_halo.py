@@ -1,6 +1,9 @@
 """The generator's convolutions and weight gradients over halo tiles, at every
 channel count they are compiled for and at grids whose planes are smaller
-than, not a multiple of, and several times a tile.
+than, not a multiple of, and several times a tile.  In the last case the halo
+tile of the finest level's 128-channel layers does not fit the shared memory
+(2 (128 + 2) (256 + 2 (256 + 3)) + 18 * 128 * 16 bytes and more, of 225 KB): those
+layers, forward, output and input gradient, take the im2col convolution.
 
 Weights with three terms of +-1 or +-1/2 per output, FiLM tables of eighths and
 r = +-1/2: every FP32 sum of the forward pass is exact up to its last bit, so
@@ -42,6 +45,7 @@ def exact_params(cfg, rng):
     (16, 48, 8, [48, 96, 128, 112], 128),  # long in y
     (128, 8, 8, [112, 16, 16, 48], 48),    # the longest rows that two buffers hold
     (64, 48, 8, [32, 48, 64, 32], 16),     # planes of the default grid
+    (256, 8, 8, [16, 16, 32, 128], 16),    # 128 channels of a row too long for the shared memory
 ])
 def test_halo_tiles_match_oracle(nx, ny, nz, channels, latent):
     from powerllel_channel_sycl_b200.learned import Generator, config
