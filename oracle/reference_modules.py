@@ -25,7 +25,7 @@ import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "_ref", "libplcref.so")
-REF_SRC = os.environ.get("PLC_REFERENCE_SRC", "/root/reference/src")
+REF_SRC = os.environ.get("PLC_REFERENCE_SRC", "")  # the reference's src/ folder
 
 FIELDS = {"u": 0, "v": 1, "w": 2, "u1": 3, "v1": 4, "w1": 5, "p": 6}
 MESH = {"dzf_global": 0, "dzf": 1, "dzf_inv": 2, "dzc": 3, "dzc_inv": 4, "dzflzi": 5,
