@@ -3,7 +3,7 @@
 
 Both solve the same systems with the same pivots in different orders of
 operations, so both are held to a solution in extended precision (FP64 form) or
-in FP64 (mixed form): the split sweep may be at most twice as far off as the
+in FP64 (mixed form): the split sweep may be a twentieth further off than the
 streaming one, plus one rounding of the result.  The sizes are the edges of the
 compiled segment lengths (4, 8 and 16 planes for 16 segments, the streaming
 sweep above 256 planes), segments left empty or short, lanes that do not fill a
@@ -72,7 +72,7 @@ def test_split_sweep_fp64(monkeypatch, nx, ny, nz):
     mask = np.ones((ny, nx), bool)
     mask[0, 0] = False
     err = {m: rel_l2(g[:, mask], ref[:, mask]) for m, g in got.items()}
-    assert err["split"] <= 2 * err["stream"] + 2.0 ** -53, err
+    assert err["split"] <= 1.05 * err["stream"] + 2.0 ** -53, err
     # the singular system of a random right-hand side: the same constant
     assert rel_l2(got["split"][:, 0, 0], got["stream"][:, 0, 0]) < 1e-9
 
@@ -115,7 +115,7 @@ def test_split_sweep_mixed(monkeypatch, nx, ny, nz):
         got[key] = np.stack([ch.download(name)[1:-1, 1:-1, 1:-1] for name in "uvw"])
         ch.close()
     err = {m: rel_l2(got[m], got["exact"]) for m in ("split", "stream")}
-    assert err["split"] <= 2 * err["stream"] + 2.0 ** -24, err
+    assert err["split"] <= 1.05 * err["stream"] + 2.0 ** -24, err
 
 
 # members whose segments have each compiled length; a column above 256 planes on
