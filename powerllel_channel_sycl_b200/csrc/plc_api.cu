@@ -684,7 +684,7 @@ int plc_create(const plc_params *prm, const double *h_dzf_global, int device, pl
       return fail(cuda_status(c, e, "fft_set_lines"));
   }
   // PLC_TRID = "split" / "tile" / "stream" pins the Thomas sweep (columns split
-  // over the threads of a block where they fit, on chip, or streamed through
+  // over the threads of a block wherever they fit, on chip, or streamed through
   // HBM; columns too tall for the split one are streamed under its pin)
   if (const char *env = getenv("PLC_TRID")) {
     if (strcmp(env, "split") != 0 && strcmp(env, "tile") != 0 && strcmp(env, "stream") != 0)

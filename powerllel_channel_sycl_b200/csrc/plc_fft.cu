@@ -3239,10 +3239,10 @@ cudaError_t fft_autotune_t(plc_ctx *c, T *const *f, size_t dev_max, int sms) {
          else
            return launch_fft_x_fwd(c, u, v, w, spec, s);
        });
-  // the Thomas sweep of columns too tall for the split one: on chip or
+  // the Thomas sweep of grids that do not take the split one: on chip or
   // streaming, timed on the spectral array (the choice changes speed, never
   // results)
-  if (c->nx % 32 == 0 && !c->trid_pinned && !trid_split_ok(c->nz)) {
+  if (c->nx % 32 == 0 && !c->trid_pinned && trid_sweep(c, sizeof(T), spec) != TRID_SPLIT) {
     float t_tile = -1.f, t_stream = -1.f;
     c->trid_tile = true;
     t_tile = time_of([&]() -> cudaError_t { return launch_trid(c, spec, s); });

@@ -108,10 +108,10 @@ struct plc_ctx {
   int fft_plan_x = 0, fft_plan_y = 0;
   // family of the forward x transform (-1: that of the backward one)
   int fft_plan_xf = -1;
-  // Thomas sweep: its columns split over the threads of a block wherever they fit
-  // (trid_split_ok), unless PLC_TRID pins a serial one; taller columns have
-  // the sweep with the columns on chip or the streaming one, as the autotuner
-  // finds; the device's shared-memory limit per block
+  // Thomas sweep: its columns split over the threads of a block where they fit and
+  // that is faster (trid_sweep), unless PLC_TRID pins a serial one; other grids
+  // have the sweep with the columns on chip or the streaming one, as the
+  // autotuner finds; the device's shared-memory limit per block
   bool trid_split = true;
   bool trid_tile = true;
   bool trid_pinned = false;  // PLC_TRID = "split", "tile" or "stream"
@@ -417,6 +417,34 @@ constexpr int kTridChunks = 8;
 inline size_t trid_tile_smem(int nz, size_t elem) {
   return (size_t)nz * 32 * elem + 8 * kTridChunks + 16;
 }
+// Whether the split sweep is the faster one for a column that fits it.  A serial
+// sweep takes a chain of 2 nz dependent operations however few systems there
+// are (FP64 0.19 us a plane, mixed 0.38), until their number sets its time; the
+// split one takes 7 us at least and 16 segments of one length, compiled for 4,
+// 8 or 16 planes, whatever nz is.  So the split sweep pays where the segments
+// are whole (64, 128 and 256 planes: 768 x 384 x 256 FP64 0.41 -> 0.30 ms, mixed
+// 0.23 -> 0.17), and otherwise for up to so many systems per SM.  On either side
+// of the lines, serial and split sweep in us:
+//   FP64   256 x 128 x 110  26, 22    384 x 192 x 110   34,  38
+//          128 x  96 x  18   9,  8    192 x 144 x  18    9,  11
+//   mixed  384 x 288 x 194 114, 102   512 x 384 x 194  125, 147
+//          768 x 384 x  80  73,  68  1024 x 512 x  80  125, 128
+//          512 x 288 x  30  25,  21   512 x 288 x  18   16,  19
+//          192 x 144 x  18  14,  10   384 x 192 x  18   14,  16
+// A rule and not a timing, because the two differ by rounding: a grid's results
+// do not depend on how a context was tuned.
+inline bool trid_split_pays(const plc_ctx *c, size_t elem) {
+  const int nz = c->nz;
+  if (nz == kTridSplitMax / 4 || nz == kTridSplitMax / 2 || nz == kTridSplitMax) return true;
+  long long per_sm;
+  if (elem == sizeof(double))
+    per_sm = nz < 32 ? 96 : 224;
+  else if (nz > 24 && nz < kTridSplitMax / 4)  // the FP32 streaming sweep loads 24 planes at once
+    return true;
+  else
+    per_sm = nz <= 24 ? 224 : (nz < kTridSplitMax / 2 ? 2048 : 1024);
+  return (long long)c->nx * c->ny <= per_sm * c->device_sms;
+}
 // The Thomas sweep of a solve of the spectral array `var` of elem-byte elements.
 // The split sweep loads pairs of elements and the on-chip sweep rows by bulk
 // copies from 16-byte boundaries; any other array takes the streaming sweep,
@@ -425,7 +453,9 @@ inline size_t trid_tile_smem(int nz, size_t elem) {
 enum TridSweep { TRID_SPLIT, TRID_TILE, TRID_STREAM };
 inline TridSweep trid_sweep(const plc_ctx *c, size_t elem, const void *var) {
   const size_t at = reinterpret_cast<size_t>(var);
-  if (c->trid_split && trid_split_ok(c->nz) && at % (2 * elem) == 0) return TRID_SPLIT;
+  if (c->trid_split && trid_split_ok(c->nz) && at % (2 * elem) == 0 &&
+      (c->trid_pinned || trid_split_pays(c, elem)))
+    return TRID_SPLIT;
   if (c->trid_tile && c->nx % 32 == 0 && at % 16 == 0 &&
       trid_tile_smem(c->nz, elem) <= c->trid_smem_max)
     return TRID_TILE;

@@ -22,9 +22,11 @@
 // the pivots and every multiplier, which is what keeps the instruction count
 // below the memory time.
 //
-// What bounds it: memory.  Every value is read once and written once, all loads
-// of a thread are in flight at once, and several blocks per SM overlap their
-// loads, sweeps and stores.  Measured against the serial streaming sweep, per
+// What bounds it: memory, where the segments are whole.  Every value is read once
+// and written once, all loads of a thread are in flight at once, and several
+// blocks per SM overlap their loads, sweeps and stores.  Segments that are not
+// whole leave threads idle and pay the guarded code, so large planes of other
+// columns stay with the serial sweeps (trid_split_pays).  Measured against the serial streaming sweep, per
 // solve: FP64 768 x 384 x 256 0.42 -> 0.31 ms (a copy in the same access pattern
 // takes 0.20), 256 x 192 x 128 28 -> 22 us, 128 x 64 x 64 10 -> 3 us; mixed 0.23 ->
 // 0.17 ms, 52 -> 16 us, 22 -> 3 us.  Tried and slower at the large size: one

@@ -1,5 +1,5 @@
 """The Thomas sweep with its columns split over the threads of a block
-(PLC_TRID=split, the default) against the streaming sweep.
+(PLC_TRID=split, and the default where it pays) against the streaming sweep.
 
 Both solve the same systems with the same pivots in different orders of
 operations, so both are held to a solution in extended precision (FP64 form) or
@@ -120,10 +120,11 @@ def test_split_sweep_mixed(monkeypatch, nx, ny, nz):
 
 # members whose segments have each compiled length; a column above 256 planes on
 # chip or streamed as tuned, and one that only the streaming sweep takes, beside
-# short ones; a grid whose own solves take a lane per pair in both directions
+# short ones; a grid whose own solves take a lane per pair in both directions,
+# and one with too few planes for the split sweep to pay
 ENSEMBLES = [[(32, 24, 16), (36, 24, 54), (32, 32, 130), (24, 24, 250)],
              [(32, 24, 16), (32, 32, 258), (36, 24, 54), (24, 24, 300)],
-             [(512, 288, 10), (32, 24, 16), (24, 24, 258)]]
+             [(512, 288, 64), (32, 24, 16), (512, 288, 10), (24, 24, 258)]]
 
 
 @pytest.mark.parametrize("chains", [1, 2])
