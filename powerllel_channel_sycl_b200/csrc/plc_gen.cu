@@ -706,7 +706,9 @@ bool wgrad_halo(plc_gen *gn, Shape s, const bf16 *dy, const bf16 *x, float *dw, 
 // weight gradient on the tensor cores: over halo tiles, else per tap with
 // M = co (zero-padded to 128), N = ci
 int wgrad(plc_gen *gn, Shape s, const bf16 *dy, const bf16 *x, float *dw, int ci, int co) {
+  // (of more latent channels only the forward pass is offered, on any grid)
   if (co > 128 || co % 16) return gen_error(gn, PLC_ERR_ARG, "weight gradient: co must be a multiple of 16 <= 128");
+  if (ci > 128 || ci % 16) return gen_error(gn, PLC_ERR_ARG, "weight gradient: ci must be a multiple of 16 <= 128");
   cudaError_t e;
   bool done = false;
   switch (co) {

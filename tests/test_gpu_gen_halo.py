@@ -75,3 +75,19 @@ def test_halo_tiles_match_oracle(nx, ny, nz, channels, latent):
             assert rel(grad[off:off + n], gref[off:off + n]) < 1e-3, (ci, co, lv)
         off += n
     assert rel(grad, gref) < 1e-3
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(8, 8, 8), (64, 16, 16), (24, 24, 8)])
+def test_more_latent_channels_forward_only(nx, ny, nz):
+    """Above 128 latent channels the forward pass runs and gradients are refused,
+    whether the coarsest grid admits halo tiles or not."""
+    from powerllel_channel_sycl_b200 import PlcError
+    from powerllel_channel_sycl_b200.learned import Generator, config
+    g = Generator(config(nx=nx, ny=ny, nz=nz, channels=[16, 16, 16, 16], latent_channels=144, batch=1,
+                         seed=3))
+    g.set_targets([180.0], np.full((1, nz, go.NSTAT), 0.1))
+    assert np.isfinite(g.forward([180.0], seed=7)).all()
+    with pytest.raises(PlcError, match="weight gradient"):
+        g.loss_grad(np.array([0], np.int32), [180.0], seed=7)
+    with pytest.raises(PlcError, match="weight gradient"):
+        g.train(1)
