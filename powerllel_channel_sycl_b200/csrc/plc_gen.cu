@@ -542,20 +542,29 @@ void gen_free(plc_gen *gn) {
 // dynamic shared memory that a block may take beside its static kilobyte
 constexpr size_t kSmemMax = 225 * 1024;
 
-// Output channels per block of a halo-tile convolution: the most (of N and the
-// parts of it that are multiples of 16) of which two blocks fit an SM and whose
-// blocks fill the device -- fewer channels read the input tile again --, else
-// the fewest if one block fits, else 0.
+// Output channels per block of a halo-tile convolution, or 0 for the im2col one:
+// the most (of n and the parts of it that are multiples of 16) of which two
+// blocks fit an SM and whose blocks fill the device -- fewer channels read the
+// input tile again.  Where two blocks do not fit, one block per SM does not
+// overlap its copies with another's MMAs: worth it for up to four parts (forward
+// pass with two layers of the given channels at the finest level, im2col and halo:
+// 80 channels of 192 x 64 x 32 2.8 and 1.4 ms in one part, 128 of 128 x 64 x 32 3.2 and
+// 2.9 in four), not for more (80 of 256 x 64 x 16 2.0 and 2.5 in five, 128 of 192 x
+// 64 x 32 4.7 and 7.3 in eight).  A grid with less than two im2col blocks per SM
+// takes the fewest channels that fit (112 of 64 x 48 x 8 0.54 and 0.47 ms).
 int halo_channels(int sms, Shape s, int ci, int n) {
   const long long tiles = (long long)((s.Y * (s.X + 2) + kHaloM - 1) / kHaloM) * s.B * s.Z;
-  int least = 0;
+  int one = 0, least = 0;
   for (int parts = 1; parts <= n / 16; ++parts) {
     if (n % parts || n / parts % 16) continue;
     const int nb = n / parts;
-    if (halo_smem(s.X, ci, nb) <= kSmemMax / 2 && tiles * parts >= sms) return nb;
-    if (halo_smem(s.X, ci, nb) <= kSmemMax) least = nb;
+    if (halo_smem(s.X, ci, nb) > kSmemMax) continue;
+    least = nb;
+    if (tiles * parts < sms) continue;
+    if (halo_smem(s.X, ci, nb) <= kSmemMax / 2) return nb;
+    if (!one && parts <= 4) one = nb;
   }
-  return least;
+  return one ? one : (s.voxels() < 2ll * kTcM * sms ? least : 0);
 }
 
 template <int NB>

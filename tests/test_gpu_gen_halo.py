@@ -1,9 +1,10 @@
 """The generator's convolutions and weight gradients over halo tiles, at every
 channel count they are compiled for and at grids whose planes are smaller
-than, not a multiple of, and several times a tile.  In the last case the halo
+than, not a multiple of, and several times a tile.  In the case of 256 cells the halo
 tile of the finest level's 128-channel layers does not fit the shared memory
 (2 (128 + 2) (256 + 2 (256 + 3)) + 18 * 128 * 16 bytes and more, of 225 KB): those
-layers, forward, output and input gradient, take the im2col convolution.
+layers, forward, output and input gradient, take the im2col convolution, as do
+the 112-channel layers of the last case, whose tiles would be read in seven parts.
 
 Weights with three terms of +-1 or +-1/2 per output, FiLM tables of eighths and
 r = +-1/2: every FP32 sum of the forward pass is exact up to its last bit, so
@@ -46,6 +47,8 @@ def exact_params(cfg, rng):
     (128, 8, 8, [112, 16, 16, 48], 48),    # the longest rows that two buffers hold
     (64, 48, 8, [32, 48, 64, 32], 16),     # planes of the default grid
     (256, 8, 8, [16, 16, 32, 128], 16),    # 128 channels of a row too long for the shared memory
+    (64, 16, 8, [128, 96, 64, 128], 16),   # one block per SM, 32 of 128 channels each
+    (64, 40, 8, [128, 96, 64, 112], 16),   # 112 channels: seven blocks would read each tile
 ])
 def test_halo_tiles_match_oracle(nx, ny, nz, channels, latent):
     from powerllel_channel_sycl_b200.learned import Generator, config
