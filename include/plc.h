@@ -390,9 +390,13 @@ int plc_get_stream(plc_ctx *ctx, void **stream);
  * ms_per_kernel[0..count-1]; *count receives the number of kernels per step
  * (at most 16).  Used for per-kernel roofline figures; advances the state. */
 int plc_profile_step(plc_ctx *ctx, int nsteps, float *ms_per_kernel, int *count);
-/* Name of kernel i of the fused step of the FP64 form (static string). */
+/* Name of kernel i of the fused step of the FP64 form (static string) of a
+ * channel that is not forced in x alone.  One that is, and the mixed form, have
+ * fewer kernels with other names: name those of plc_profile_step with
+ * plc_step_kernel_name_ctx. */
 const char *plc_step_kernel_name(int i);
-/* Name of kernel i of the context's fused step (either form). */
+/* Name of kernel i of the context's fused step (either form), as plc_profile_step
+ * numbers them. */
 const char *plc_step_kernel_name_ctx(const plc_ctx *ctx, int i);
 
 /* ---- host-only helpers (no GPU needed) ---- */
