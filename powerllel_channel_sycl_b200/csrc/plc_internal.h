@@ -421,28 +421,33 @@ inline size_t trid_tile_smem(int nz, size_t elem) {
 // sweep takes a chain of 2 nz dependent operations however few systems there
 // are (FP64 0.19 us a plane, mixed 0.38), until their number sets its time; the
 // split one takes 7 us at least and 16 segments of one length, compiled for 4,
-// 8 or 16 planes, whatever nz is.  So the split sweep pays where the segments
-// are whole (64, 128 and 256 planes: 768 x 384 x 256 FP64 0.41 -> 0.30 ms, mixed
-// 0.23 -> 0.17), and otherwise for up to so many systems per SM.  On either side
-// of the lines, serial and split sweep in us:
-//   FP64   256 x 128 x 110  26, 22    384 x 192 x 110   34,  38
-//          128 x  96 x  18   9,  8    192 x 144 x  18    9,  11
-//   mixed  384 x 288 x 194 114, 102   512 x 384 x 194  125, 147
-//          768 x 384 x  80  73,  68  1024 x 512 x  80  125, 128
-//          512 x 288 x  30  25,  21   512 x 288 x  18   16,  19
-//          192 x 144 x  18  14,  10   384 x 192 x  18   14,  16
+// 8 or 16 planes (64, 128 or 256 in all), whatever nz is.  So the split sweep pays
+// where the segments are whole (768 x 384 x 256 FP64 0.41 -> 0.30 ms, mixed 0.23 ->
+// 0.17), in FP64 nearly whole, and otherwise for up to so many systems per SM.
+// On either side of the lines, a whole step with the serial and with the split
+// sweep, in us:
+//   FP64   144 x  96 x  30   74,   72    256 x 128 x  16   72,   76
+//          216 x 192 x 110  373,  368    256 x 192 x 150  517,  528
+//          512 x 384 x 110 1505, 1478    512 x 384 x  54  738,  744
+//   mixed  256 x 128 x  18   68,   66    384 x 192 x  18   92,   95
+//          512 x 288 x 218 1354, 1344    512 x 384 x 218 1694, 1713
+//          768 x 384 x  74  868,  861   1024 x 512 x  90 1974, 1988
 // A rule and not a timing, because the two differ by rounding: a grid's results
 // do not depend on how a context was tuned.
 inline bool trid_split_pays(const plc_ctx *c, size_t elem) {
   const int nz = c->nz;
-  if (nz == kTridSplitMax / 4 || nz == kTridSplitMax / 2 || nz == kTridSplitMax) return true;
+  const int whole = nz <= kTridSplitMax / 4 ? kTridSplitMax / 4
+                    : nz <= kTridSplitMax / 2 ? kTridSplitMax / 2
+                                              : kTridSplitMax;
   long long per_sm;
-  if (elem == sizeof(double))
-    per_sm = nz < 32 ? 96 : 224;
-  else if (nz > 24 && nz < kTridSplitMax / 4)  // the FP32 streaming sweep loads 24 planes at once
-    return true;
-  else
+  if (elem == sizeof(double)) {
+    if (32 * nz > 27 * whole) return true;
+    per_sm = nz < 32 ? 96 : 288;
+  } else {
+    // (the FP32 streaming sweep loads 24 planes at once)
+    if (nz == whole || (nz > 24 && nz < kTridSplitMax / 4)) return true;
     per_sm = nz <= 24 ? 224 : (nz < kTridSplitMax / 2 ? 2048 : 1024);
+  }
   return (long long)c->nx * c->ny <= per_sm * c->device_sms;
 }
 // The Thomas sweep of a solve of the spectral array `var` of elem-byte elements.

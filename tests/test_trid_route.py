@@ -83,11 +83,12 @@ def test_aligned_arrays(sweeps):
 RULE = [((32, 24, 16), True, True), ((64, 48, 48), True, True), ((162, 108, 90), True, True),
         ((128, 96, 2), True, True), ((192, 144, 18), False, True), ((384, 192, 18), False, False),
         ((512, 288, 24), False, False), ((512, 288, 26), False, True), ((192, 144, 30), False, True),
-        ((256, 128, 32), True, True), ((256, 192, 32), False, True), ((256, 192, 130), False, True),
-        ((512, 288, 250), False, True), ((512, 384, 130), False, False), ((512, 384, 110), False, True),
-        ((768, 384, 62), False, True), ((768, 384, 110), False, True), ((768, 384, 130), False, False),
-        ((1024, 512, 62), False, True), ((1024, 512, 66), False, False),
-        ((1024, 512, 126), False, False)] + [((nx, nx // 2, nz), True, True)
+        ((256, 128, 32), True, True), ((216, 192, 38), True, True), ((256, 192, 38), False, True),
+        ((256, 192, 130), False, True), ((512, 288, 216), False, True), ((512, 288, 218), True, True),
+        ((512, 384, 130), False, False), ((512, 384, 54), False, True), ((512, 384, 56), True, True),
+        ((768, 384, 108), False, True), ((768, 384, 110), True, True), ((768, 384, 130), False, False),
+        ((768, 384, 250), True, False), ((1024, 512, 66), False, False),
+        ((1024, 512, 126), True, False)] + [((nx, nx // 2, nz), True, True)
                                              for nx in (64, 768, 1536) for nz in (64, 128, 256)]
 
 
